@@ -97,3 +97,76 @@ Q4_HD uint32_t q4_rows_plan(uint32_t cpt, uint32_t tiles, uint32_t sm_count, uin
     if (cost_out) *cost_out = best_cost;
     return best;
 }
+
+// ---- tensor-core GEMM (q4_gemm_tc.cu): how a launch is cut ----
+
+struct Q4GemmPlan {
+    uint32_t bn;            // activation rows per tile: a multiple of 32, at most 256
+    uint32_t accs, stages;  // accumulators and A stages in TMEM: accs * bn + 64 * stages <= 512 columns
+    uint32_t tiles, tiles_m;  // output tiles of 256 weight rows x bn activation rows; tiles along m
+    uint32_t workers;       // CTA pairs
+    uint32_t full_rounds;   // whole tiles per worker ...
+    uint32_t tail_workers;  // ... and workers that share the K stages of the tiles left over
+    uint64_t partial_floats;  // scratch for the parts of tiles that are cut between workers
+    uint32_t counters;
+};
+
+// row tiles of an n-row projection: 256 weight rows of one tensor, or (pair mode) 128 gate rows and the same up rows
+Q4_HD uint32_t q4_gemm_row_tiles(uint32_t n, uint32_t pair) { return pair ? (n + 127u) / 128u : (n + 255u) / 256u; }
+
+// K stages of 128 inputs (two affine groups)
+Q4_HD uint32_t q4_gemm_k_stages(uint32_t k) { return (k / 64u + 1u) / 2u; }
+
+// The plan with the smallest estimate, in SM cycles. A stage of bn activation rows takes 4 bn cycles of MMA, but no
+// less than the ~600 in which an SM's warps expand 128 x 128 weights; a tile's epilogue takes about 20 cycles a column
+// and is hidden when there are two accumulators (bn <= 128); every part of a tile that is cut costs another pass over
+// bn columns, and the last one adds them all up.
+// Candidates: the fewest activation tiles and up to two more (narrower tiles waste less on ragged m); whole tiles for
+// everybody, or all but the last one or two rounds whole and the rest cut along K over all workers, or over fewer
+// workers when there is little to cut.
+inline void q4_gemm_plan(uint32_t m, uint32_t k, uint32_t row_tiles, uint32_t pairs, Q4GemmPlan *plan) {
+    const uint32_t ks = q4_gemm_k_stages(k);
+    double best = 0.0;
+    bool have = false;
+    for (uint32_t tm = (m + 255u) / 256u, tries = 0; tries < 3u; ++tm, ++tries) {
+        const uint32_t bn = (((m + tm - 1u) / tm) + 31u) & ~31u;
+        if (tries > 0 && bn < 96u) break;
+        const uint32_t tiles_m = (m + bn - 1u) / bn, tiles = row_tiles * tiles_m;
+        const uint32_t accs = bn <= 128u ? 2u : 1u;
+        const uint32_t stages = (512u - accs * bn) / 64u < 8u ? (512u - accs * bn) / 64u : 8u;
+        const double stage = 4.0 * bn > 600.0 ? 4.0 * bn : 600.0, epilogue = 20.0 * bn + 1000.0, shown = accs == 2u ? 0.0 : epilogue;
+        auto consider = [&](uint32_t workers, uint32_t rounds, uint32_t tail_workers) {
+            const uint32_t whole = rounds * workers < tiles ? rounds * workers : tiles, rest = tiles - whole;
+            double cost = rounds * (ks * stage + shown) + epilogue;
+            if (rest) {
+                const uint64_t units = (uint64_t)rest * ks;
+                const double run = (double)((units + tail_workers - 1u) / tail_workers);
+                const double parts = ks / run < 1.0 ? 2.0 : ks / run + 1.0;  // contributors of a tile
+                cost += run * stage + 2000.0 + epilogue + parts * bn * 10.0;
+            }
+            if (have && cost >= best) return;
+            have = true;
+            best = cost;
+            plan->bn = bn;
+            plan->accs = accs;
+            plan->stages = stages;
+            plan->tiles = tiles;
+            plan->tiles_m = tiles_m;
+            plan->workers = workers;
+            plan->full_rounds = rounds;
+            plan->tail_workers = rest ? tail_workers : 0u;
+            plan->partial_floats = rest ? (uint64_t)tail_workers * 2u * bn * 256u : 0u;
+            plan->counters = rest * 8u;
+        };
+        if (tiles <= pairs) {
+            consider(tiles, 1u, 0u);
+            for (uint32_t parts = 2; tiles * (parts - 1u) < pairs && parts <= ks; ++parts) {
+                const uint32_t w = tiles * parts < pairs ? tiles * parts : pairs;
+                if ((uint64_t)w <= (uint64_t)tiles * ks) consider(w, 0u, w);
+            }
+        } else {
+            consider(pairs, (tiles + pairs - 1u) / pairs, 0u);
+            if (tiles % pairs) consider(pairs, tiles / pairs - 1u, pairs);
+        }
+    }
+}

@@ -148,6 +148,13 @@ __device__ __forceinline__ uint32_t ldg_bf16_bits(const uint8_t *p) {
     return (uint32_t)__ldg(p) | ((uint32_t)__ldg(p + 1) << 8);
 }
 
+// Programmatic dependent launch: a kernel launched with the programmatic attribute may start while the kernel before it
+// in the stream still runs. The wait returns once that kernel has finished and its writes are visible (at once when the
+// kernel was launched the ordinary way). The second call lets the next kernel start; it is made after the wait, so
+// that whatever a dependent kernel reads ahead of its own wait was written before the kernel in front of it began.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Constants of the nibble conversion, held in registers the compiler cannot see through so that
 // mask-and-or stays one three-input logic instruction (with two immediates it becomes two).
 struct Magic {

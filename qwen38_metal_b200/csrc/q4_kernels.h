@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "q4_decomp.h"
+
 namespace q4 {
 
 constexpr int kMaxJobs = 12;
@@ -81,6 +83,13 @@ struct RowsParams {
     unsigned long long *trace;  // optional [warps of the grid][4] globaltimer stamps (start, digits ready, first tile streamed, done)
 };
 
+// One projection of a tensor-core launch (q4_gemm_tc.cu): any byte alignment.
+struct GemmJob {
+    const uint8_t *w, *s, *b;
+    float *out;            // [m][n] fp32
+    uint32_t n;            // output rows
+};
+
 }  // namespace q4
 
 extern "C" {
@@ -103,16 +112,10 @@ cudaError_t q4k_dequantize_row(const uint8_t *w, const uint8_t *s, const uint8_t
                                cudaStream_t stream);
 
 cudaError_t q4k_gemm_prepare_x(const void *x, int x_is_f32, uint64_t elements, uint16_t *xp, cudaStream_t stream);
-uint32_t q4k_gemm_tile_m(uint32_t m);
-uint32_t q4k_gemm_k_splits(uint32_t m, uint32_t n, uint32_t k, uint32_t sm_count, uint32_t *split_blocks);
-cudaError_t q4k_gemm_tc(const uint16_t *xp, uint32_t m, uint32_t k, const uint8_t *w, const uint8_t *s, const uint8_t *b,
-                        uint32_t n, float *out, uint32_t out_stride, int accumulate, int *error_flag, uint32_t sm_count,
-                        float *parts, cudaStream_t stream);
-
+cudaError_t q4k_gemm_tc(const Q4GemmPlan *plan, const uint16_t *xp, uint32_t m, uint32_t k, const q4::GemmJob *jobs, uint32_t n_jobs,
+                        uint16_t *h_out, uint32_t h_stride, int accumulate, int *error_flag, float *partials, unsigned int *counters,
+                        cudaStream_t stream);
 int q4k_gemm_pair_supported(const uint8_t *w_gate, const uint8_t *w_up);
-cudaError_t q4k_gemm_tc_pair(const uint16_t *xp, uint32_t m, uint32_t k, const uint8_t *wg, const uint8_t *sg, const uint8_t *bg,
-                             const uint8_t *wu, const uint8_t *su, const uint8_t *bu, uint32_t n, uint16_t *h_out, uint32_t h_stride,
-                             int *error_flag, uint32_t sm_count, cudaStream_t stream);
 
 cudaError_t q4k_synth_q4(uint64_t seed, uint64_t tensor, float sigma, uint64_t row0, uint64_t rows, uint32_t k,
                          uint8_t *w, uint8_t *s, uint8_t *b, cudaStream_t stream);

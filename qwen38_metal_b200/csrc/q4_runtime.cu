@@ -131,7 +131,8 @@ struct q4b_runtime {
     uint32_t gemv_ctas[3][2] = {{0, 0}, {0, 0}, {0, 0}};  // [column tiles][aligned] resident warps per SM
     uint32_t max_workers = 0;
     std::vector<void *> arenas, peer_arenas;
-    Pool trace, gemm_x, gemm_parts, error_flag;
+    Pool trace, gemm_x, gemm_parts, gemm_counters, error_flag;
+    uint64_t gemm_failures_seen = 0;  // rt->failures when the GEMM's tile counters were last known to be zero
     uint32_t gemm_min_m = 16;  // activation rows from which the tensor-core GEMM takes over (when the short-batch kernel does not apply)
     uint32_t rows_max_m = 16;  // activation rows per launch of the short-batch kernel (0: never use it)
     uint32_t chain_offset_cost = 140;  // per cent: cost of a byte-offset projection's chunk against an aligned one (decode chain)
@@ -424,25 +425,49 @@ int launch_streaming(q4b_runtime *rt, const void *x_dev, int x_dtype, uint32_t m
     return Q4B_OK;
 }
 
-// Tensor-core path: activations to bf16 once, then one tcgen05 GEMM launch per projection.
+// One tensor-core launch over up to kMaxJobs projections (or the fused gate/up pair when h_out is given).
+int launch_gemm(q4b_runtime *rt, const uint16_t *xp, uint32_t m, uint32_t k, const Resolved *jobs, uint32_t n_jobs, float *const *outs,
+                uint16_t *h_out, uint32_t h_stride, uint32_t flags, cudaStream_t stream) {
+    q4::GemmJob list[q4::kMaxJobs];
+    uint32_t row_tiles = 0;
+    uint64_t rows = 0;
+    for (uint32_t i = 0; i < n_jobs; ++i) {
+        list[i] = q4::GemmJob{jobs[i].w, jobs[i].s, jobs[i].b, outs ? outs[i] : nullptr, jobs[i].n};
+        if (!h_out || i == 0) row_tiles += q4_gemm_row_tiles(jobs[i].n, h_out ? 1u : 0u);
+        rows += jobs[i].n;
+    }
+    Q4GemmPlan plan;
+    q4_gemm_plan(m, k, row_tiles, (uint32_t)rt->sm_count / 2u, &plan);
+    if (plan.counters) {
+        Q4B_CUDA(rt->gemm_parts.ensure(plan.partial_floats * 4), "partial tile scratch");
+        const size_t had = rt->gemm_counters.capacity;
+        Q4B_CUDA(rt->gemm_counters.ensure((size_t)plan.counters * 4), "tile counter scratch");
+        // (put back to zero by the kernel itself, like the short-batch kernel's)
+        if (rt->gemm_counters.capacity != had || rt->gemm_failures_seen != rt->failures) {
+            Q4B_CUDA(cudaMemsetAsync(rt->gemm_counters.ptr, 0, rt->gemm_counters.capacity, stream), "tile counter reset");
+            rt->gemm_failures_seen = rt->failures;
+        }
+    }
+    if (int st = profile_open(rt, stream)) return st;
+    Q4B_CUDA(q4k_gemm_tc(&plan, xp, m, k, list, n_jobs, h_out, h_stride, (flags & Q4B_FLAG_ACCUMULATE) ? 1 : 0, (int *)rt->error_flag.ptr,
+                         (float *)rt->gemm_parts.ptr, (unsigned int *)rt->gemm_counters.ptr, stream),
+             "q4_gemm_tc launch");
+    rt->launches++;
+    const uint64_t out_bytes = h_out ? (uint64_t)m * jobs[0].n * 2 : (uint64_t)m * rows * 4;
+    return profile_close(rt, stream, rows * (k / 2 + (uint64_t)(k / 64) * 4) + (uint64_t)m * k * 2 + out_bytes, 2ull * m * rows * k);
+}
+
+// Tensor-core path: activations to bf16 once, then one tcgen05 launch for all projections (twelve at a time).
 int enqueue_gemm(q4b_runtime *rt, const void *x_dev, int x_dtype, uint64_t m, uint64_t k, const std::vector<Resolved> &jobs,
                  float *const *outs, uint32_t flags, cudaStream_t stream) {
     Q4B_CUDA(rt->gemm_x.ensure((size_t)m * k * 2), "activation scratch");
     Q4B_CUDA(q4k_gemm_prepare_x(x_dev, x_dtype == Q4B_F32 ? 1 : 0, m * k, (uint16_t *)rt->gemm_x.ptr, stream),
              "q4_gemm_prepare_x launch");
     rt->launches++;
-    for (size_t i = 0; i < jobs.size(); ++i) {
-        uint32_t split_blocks = 0;
-        const uint32_t splits = q4k_gemm_k_splits((uint32_t)m, jobs[i].n, (uint32_t)k, (uint32_t)rt->sm_count, &split_blocks);
-        if (splits > 1) Q4B_CUDA(rt->gemm_parts.ensure((size_t)splits * m * jobs[i].n * 4), "partial output scratch");
-        if (int st = profile_open(rt, stream)) return st;
-        Q4B_CUDA(q4k_gemm_tc((const uint16_t *)rt->gemm_x.ptr, (uint32_t)m, (uint32_t)k, jobs[i].w, jobs[i].s, jobs[i].b, jobs[i].n,
-                             outs[i], jobs[i].n, (flags & Q4B_FLAG_ACCUMULATE) ? 1 : 0, (int *)rt->error_flag.ptr,
-                             (uint32_t)rt->sm_count, (float *)rt->gemm_parts.ptr, stream),
-                 "q4_gemm_tc launch");
-        rt->launches++;
-        const uint64_t bytes = (uint64_t)jobs[i].n * (k / 2 + (k / 64) * 4) + m * k * 2 + m * jobs[i].n * 4;
-        if (int st = profile_close(rt, stream, bytes, 2ull * m * jobs[i].n * k)) return st;
+    for (size_t j0 = 0; j0 < jobs.size(); j0 += q4::kMaxJobs) {
+        const uint32_t nj = (uint32_t)std::min(jobs.size() - j0, (size_t)q4::kMaxJobs);
+        if (int st = launch_gemm(rt, (const uint16_t *)rt->gemm_x.ptr, (uint32_t)m, (uint32_t)k, &jobs[j0], nj, outs + j0, nullptr, 0, flags, stream))
+            return st;
     }
     return Q4B_OK;
 }
@@ -703,7 +728,7 @@ extern "C" void q4b_runtime_destroy(q4b_runtime *rt) {
         if (s.ptr) cudaFree(s.ptr);
     for (void *p : rt->peer_arenas) cudaIpcCloseMemHandle(p);
     for (void *p : rt->arenas) cudaFree(p);
-    Pool *pools[] = {&rt->rows_partials, &rt->rows_counters, &rt->gemm_x, &rt->gemm_parts, &rt->error_flag, &rt->trace, &rt->x_in, &rt->xp, &rt->xsum, &rt->row_inv, &rt->partials, &rt->counters, &rt->logits, &rt->amax_v,
+    Pool *pools[] = {&rt->rows_partials, &rt->rows_counters, &rt->gemm_x, &rt->gemm_parts, &rt->gemm_counters, &rt->error_flag, &rt->trace, &rt->x_in, &rt->xp, &rt->xsum, &rt->row_inv, &rt->partials, &rt->counters, &rt->logits, &rt->amax_v,
                      &rt->amax_i, &rt->tokens, &rt->gate, &rt->up, &rt->hidden};
     for (Pool *p : pools) p->release();
     for (Pool &p : rt->outs) p.release();
@@ -1111,21 +1136,11 @@ extern "C" int q4b_mlp_batch_device(q4b_runtime *rt, const void *x_dev, int x_dt
         Q4B_CUDA(rt->gemm_x.ensure((size_t)m * k * 2), "activation scratch");
         Q4B_CUDA(rt->hidden.ensure((size_t)m * inter * 2), "hidden buffer");
         Q4B_CUDA(q4k_gemm_prepare_x(x_dev, x_dtype == Q4B_F32 ? 1 : 0, m * k, (uint16_t *)rt->gemm_x.ptr, s), "q4_gemm_prepare_x launch");
-        if (int st = profile_open(rt, s)) return st;
-        Q4B_CUDA(q4k_gemm_tc_pair((const uint16_t *)rt->gemm_x.ptr, (uint32_t)m, (uint32_t)k, gu[0].w, gu[0].s, gu[0].b, gu[1].w, gu[1].s,
-                                  gu[1].b, (uint32_t)inter, (uint16_t *)rt->hidden.ptr, (uint32_t)inter, (int *)rt->error_flag.ptr,
-                                  (uint32_t)rt->sm_count, s),
-                 "q4_gemm_tc pair launch");
-        if (int st = profile_close(rt, s, 2 * inter * (k / 2 + (k / 64) * 4) + m * k * 2 + m * inter * 2, 4ull * m * inter * k)) return st;
-        uint32_t split_blocks = 0;
-        const uint32_t splits = q4k_gemm_k_splits((uint32_t)m, dn[0].n, (uint32_t)inter, (uint32_t)rt->sm_count, &split_blocks);
-        if (splits > 1) Q4B_CUDA(rt->gemm_parts.ensure((size_t)splits * m * dn[0].n * 4), "partial output scratch");
-        if (int st = profile_open(rt, s)) return st;
-        Q4B_CUDA(q4k_gemm_tc((const uint16_t *)rt->hidden.ptr, (uint32_t)m, (uint32_t)inter, dn[0].w, dn[0].s, dn[0].b, dn[0].n, out_dev,
-                             dn[0].n, 0, (int *)rt->error_flag.ptr, (uint32_t)rt->sm_count, (float *)rt->gemm_parts.ptr, s),
-                 "q4_gemm_tc launch");
-        rt->launches += 3;
-        return profile_close(rt, s, (uint64_t)dn[0].n * (inter / 2 + (inter / 64) * 4) + m * inter * 2 + m * dn[0].n * 4, 2ull * m * dn[0].n * inter);
+        rt->launches++;
+        if (int st = launch_gemm(rt, (const uint16_t *)rt->gemm_x.ptr, (uint32_t)m, (uint32_t)k, gu.data(), 2, nullptr, (uint16_t *)rt->hidden.ptr,
+                                 (uint32_t)inter, 0, s))
+            return st;
+        return launch_gemm(rt, (const uint16_t *)rt->hidden.ptr, (uint32_t)m, (uint32_t)inter, dn.data(), 1, &out_dev, nullptr, 0, 0, s);
     }
     Q4B_CUDA(rt->gate.ensure((size_t)m * inter * 4), "gate buffer");
     Q4B_CUDA(rt->up.ensure((size_t)m * inter * 4), "up buffer");
@@ -1912,7 +1927,12 @@ extern "C" int q4b_describe_dispatch(q4b_runtime *rt, int x_dtype, uint64_t m, u
         }
     }
     if (m >= rt->gemm_min_m) {
-        snprintf(text, text_len, "tensor_core_gemm (tcgen05) tile_m=%u jobs=%u", q4k_gemm_tile_m((uint32_t)m), n_jobs);
+        uint32_t row_tiles = 0;
+        for (const Resolved &r : resolved) row_tiles += q4_gemm_row_tiles(r.n, 0);
+        Q4GemmPlan plan;
+        q4_gemm_plan((uint32_t)m, (uint32_t)k, row_tiles, (uint32_t)rt->sm_count / 2u, &plan);
+        snprintf(text, text_len, "tensor_core_gemm (tcgen05, CTA pairs) tile_m=%u tiles=%u full_rounds=%u k_split_workers=%u jobs=%u", plan.bn, plan.tiles,
+                 plan.full_rounds, plan.tail_workers, n_jobs);
         return Q4B_OK;
     }
     const uint32_t rows = x_dtype == Q4B_F32 ? 2u : 8u;

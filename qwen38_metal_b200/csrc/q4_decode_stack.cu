@@ -43,12 +43,6 @@ __device__ __forceinline__ unsigned long long stack_ns() {
     return t;
 }
 
-__device__ __forceinline__ void lds_v4_keep(uint4 &v, uint32_t addr, bool pred) {
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t@q ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n\t}"
-                 : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w)
-                 : "r"(addr), "r"((uint32_t)pred)
-                 : "memory");
-}
 __device__ __forceinline__ void lds_f32_keep(float &v, uint32_t addr, bool pred) {
     asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q ld.shared.f32 %0, [%1];\n\t}" : "+f"(v) : "r"(addr), "r"((uint32_t)pred) : "memory");
 }

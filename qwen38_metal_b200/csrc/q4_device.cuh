@@ -100,6 +100,14 @@ __device__ __forceinline__ uint2 lds_v2(uint32_t smem_addr) {
     return v;
 }
 
+// keeps the registers' old contents when `pred` is false
+__device__ __forceinline__ void lds_v4_keep(uint4 &v, uint32_t addr, bool pred) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t@q ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n\t}"
+                 : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w)
+                 : "r"(addr), "r"((uint32_t)pred)
+                 : "memory");
+}
+
 // 16 bytes starting `mis` (0..15) bytes into the 32-byte window {lo, hi}
 __device__ __forceinline__ uint4 realign_16(uint4 lo, uint4 hi, uint32_t mis) {
     uint32_t w0 = lo.x, w1 = lo.y, w2 = lo.z, w3 = lo.w, w4 = hi.x, w5 = hi.y, w6 = hi.z, w7 = hi.w;

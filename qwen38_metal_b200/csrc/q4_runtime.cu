@@ -238,6 +238,13 @@ bool job_is_fast(const Resolved &r, uint32_t groups) {
     return (((uintptr_t)r.w | (uintptr_t)r.s | (uintptr_t)r.b) & 15u) == 0 && groups % 8u == 0;
 }
 
+// whether a short-batch launch needs the byte-addressed instance
+bool rows_byte_addressed(const Resolved *jobs, uint32_t n_jobs, uint32_t groups) {
+    for (uint32_t i = 0; i < n_jobs; ++i)
+        if (!job_is_fast(jobs[i], groups)) return true;
+    return false;
+}
+
 int profile_open(q4b_runtime *rt, cudaStream_t stream) {
     if (!rt->profiling) return Q4B_OK;
     if (rt->prof_used + 2 > rt->prof_events.size()) {
@@ -476,14 +483,12 @@ int enqueue_gemm(q4b_runtime *rt, const void *x_dev, int x_dtype, uint64_t m, ui
 // conditions (the caller falls back to the general streaming kernel), else a status.
 int launch_rows(q4b_runtime *rt, const void *x_dev, int x_dtype, uint32_t m, uint32_t k, const Resolved *jobs, uint32_t n_jobs,
                 float *const *outs, uint32_t flags, cudaStream_t stream) {
-    if (m < 1 || m > 16 || k % 512u != 0 || ((uintptr_t)x_dev & 15u)) return -1;
+    if (m < 1 || m > 16 || ((uintptr_t)x_dev & 15u)) return -1;
     uint32_t tiles = 0;
-    for (uint32_t i = 0; i < n_jobs; ++i) {
-        if ((((uintptr_t)jobs[i].w | (uintptr_t)jobs[i].s | (uintptr_t)jobs[i].b) & 15u) != 0 || jobs[i].n == 0) return -1;
-        tiles += (jobs[i].n + 15u) / 16u;
-    }
+    for (uint32_t i = 0; i < n_jobs; ++i) tiles += (jobs[i].n + 15u) / 16u;
+    const int mis = rows_byte_addressed(jobs, n_jobs, k / 64u) ? 1 : 0;
     uint32_t part_chunks = 0, tiles_per_warp = 1;
-    const uint32_t parts = q4k_rows_plan(m, k, tiles, (uint32_t)rt->sm_count, &part_chunks, &tiles_per_warp);
+    const uint32_t parts = q4k_rows_plan(m, k, tiles, (uint32_t)rt->sm_count, mis, &part_chunks, &tiles_per_warp);
     if (parts == 0) return -1;
     q4::RowsParams p;
     memset(&p, 0, sizeof p);
@@ -508,17 +513,20 @@ int launch_rows(q4b_runtime *rt, const void *x_dev, int x_dtype, uint32_t m, uin
     p.x_is_f32 = x_dtype == Q4B_F32 ? 1u : 0u;
     p.k = k;
     p.groups = k / 64u;
-    p.cpt = k / 128u;
+    p.cpt = (p.groups + 1u) / 2u;
+    p.byte_addressed = (uint32_t)mis;
     p.parts = parts;
     p.part_chunks = part_chunks;
     p.tiles_per_warp = tiles_per_warp;
     p.tiles = tiles;
     p.accumulate = (flags & Q4B_FLAG_ACCUMULATE) ? 1u : 0u;
-    if (parts > 1) {
-        const size_t mp = m <= 8 ? 8 : 16;
-        Q4B_CUDA(rt->rows_partials.ensure((size_t)parts * mp * tiles * 16 * 4), "partial sum scratch");
+    const uint32_t items = (tiles + tiles_per_warp - 1u) / tiles_per_warp;
+    p.run = q4_rows_run(items, part_chunks, parts, (uint32_t)rt->sm_count);
+    p.part_slots = q4_rows_part_slots(p.cpt, parts, p.run);
+    if (parts > 1 || p.part_slots > 1) {
+        Q4B_CUDA(rt->rows_partials.ensure((size_t)parts * p.part_slots * q4k_rows_padded(m) * items * tiles_per_warp * 16 * 4), "partial sum scratch");
         const size_t had = rt->rows_counters.capacity;
-        Q4B_CUDA(rt->rows_counters.ensure((size_t)tiles * 4), "tile counter scratch");
+        Q4B_CUDA(rt->rows_counters.ensure((size_t)items * 4), "tile counter scratch");
         // the counters are put back to zero by the kernel itself; after a failed command on this runtime (a launch may
         // have been cut short) and for a fresh buffer they are cleared here
         if (rt->rows_counters.capacity != had || rt->rows_failures_seen != rt->failures) {
@@ -545,18 +553,24 @@ int enqueue_matmul(q4b_runtime *rt, const void *x_dev, int x_dtype, uint64_t m, 
                    const std::vector<Resolved> &jobs, float *const *outs, uint32_t flags, cudaStream_t stream) {
     const bool want_tensor = (flags & Q4B_FLAG_TENSOR) != 0, want_stream = (flags & Q4B_FLAG_STREAM) != 0;
     const size_t esize = x_dtype == Q4B_F32 ? 4 : 2;
-    // Short batches (2 .. rows_max_m rows; any m when the caller asks for the streaming form) run on the integer
-    // tensor-core kernel when every launch of the call meets its conditions.
-    bool rows = !want_tensor && m >= 2 && rt->rows_max_m >= 2 && (want_stream || m <= rt->rows_max_m) && k % 512 == 0 &&
+    // one row, K a multiple of 512, plain output: the persistent kernel (any byte offset)
+    const bool single = m == 1 && !(flags & Q4B_FLAG_ACCUMULATE) && rt->inline_max_halfs && k % 512 == 0 && k <= rt->inline_max_halfs && k <= q4k_stack_max_k();
+    // Short batches (up to rows_max_m rows; any m when the caller asks for the streaming form) run on the integer
+    // tensor-core kernel, as do single rows that the persistent kernel does not take.
+    bool rows = !want_tensor && (m >= 2 || (!single && m < rt->gemm_min_m)) && rt->rows_max_m >= 2 && (want_stream || m <= rt->rows_max_m) &&
                 ((uintptr_t)x_dev & 15u) == 0;
-    for (size_t j = 0; j < jobs.size() && rows; ++j)
-        rows = (((uintptr_t)jobs[j].w | (uintptr_t)jobs[j].s | (uintptr_t)jobs[j].b) & 15u) == 0 && jobs[j].n != 0;
     for (size_t j0 = 0; j0 < jobs.size() && rows; j0 += q4::kMaxJobs) {
         uint32_t tiles = 0, part_chunks = 0, tw = 1;
-        for (size_t j = j0; j < jobs.size() && j < j0 + q4::kMaxJobs; ++j) tiles += (jobs[j].n + 15u) / 16u;
+        const uint32_t nj = (uint32_t)std::min(jobs.size() - j0, (size_t)q4::kMaxJobs);
+        for (size_t j = j0; j < j0 + nj; ++j) tiles += (jobs[j].n + 15u) / 16u;
+        const int mis = rows_byte_addressed(&jobs[j0], nj, (uint32_t)(k / 64)) ? 1 : 0;
         const uint32_t full = (uint32_t)(m < rt->rows_max_m ? m : rt->rows_max_m), rest = (uint32_t)(m % rt->rows_max_m);
-        rows = q4k_rows_plan(full, (uint32_t)k, tiles, (uint32_t)rt->sm_count, &part_chunks, &tw) != 0 &&
-               (m <= rt->rows_max_m || rest == 0 || q4k_rows_plan(rest, (uint32_t)k, tiles, (uint32_t)rt->sm_count, &part_chunks, &tw) != 0);
+        if (mis && !want_stream && m >= rt->gemm_min_m) {
+            rows = false;
+            break;
+        }
+        rows = q4k_rows_plan(full, (uint32_t)k, tiles, (uint32_t)rt->sm_count, mis, &part_chunks, &tw) != 0 &&
+               (m <= rt->rows_max_m || rest == 0 || q4k_rows_plan(rest, (uint32_t)k, tiles, (uint32_t)rt->sm_count, mis, &part_chunks, &tw) != 0);
     }
     if (rows) {
         for (uint64_t m0 = 0; m0 < m; m0 += rt->rows_max_m) {
@@ -574,7 +588,7 @@ int enqueue_matmul(q4b_runtime *rt, const void *x_dev, int x_dtype, uint64_t m, 
         return Q4B_OK;
     }
     if (want_tensor || (!want_stream && m >= rt->gemm_min_m)) return enqueue_gemm(rt, x_dev, x_dtype, m, k, jobs, outs, flags, stream);
-    if (m == 1 && !(flags & Q4B_FLAG_ACCUMULATE) && rt->inline_max_halfs && k % 512 == 0 && k <= rt->inline_max_halfs && k <= q4k_stack_max_k()) {
+    if (single) {
         for (size_t j0 = 0; j0 < jobs.size(); j0 += q4::kMaxJobs) {
             const uint32_t nj = (uint32_t)((jobs.size() - j0) < (size_t)q4::kMaxJobs ? (jobs.size() - j0) : (size_t)q4::kMaxJobs);
             if (int st = launch_single_row(rt, x_dev, x_dtype, (uint32_t)k, &jobs[j0], nj, outs + j0, stream)) return st;
@@ -695,6 +709,10 @@ extern "C" int q4b_runtime_create(int device_ordinal, q4b_runtime **out) {
     if (e == cudaSuccess) e = cudaMemset(rt->counters.ptr, 0, rt->counters.capacity);
     if (e == cudaSuccess) e = rt->error_flag.ensure(256);
     if (e == cudaSuccess) e = cudaMemset(rt->error_flag.ptr, 0, rt->error_flag.capacity);
+    // enough for a decode layer's projections of a few rows; larger launches grow it
+    if (e == cudaSuccess) e = rt->rows_partials.ensure((size_t)4 << 20);
+    if (e == cudaSuccess) e = rt->rows_counters.ensure(16384 * 4);
+    if (e == cudaSuccess) e = cudaMemset(rt->rows_counters.ptr, 0, rt->rows_counters.capacity);
     if (const char *unf = getenv("Q4B_MLP_UNFUSED")) rt->mlp_unfused = strtol(unf, nullptr, 10) != 0;
     if (const char *off = getenv("Q4B_NO_INLINE")) rt->inline_off = strtol(off, nullptr, 10) != 0;
     if (e == cudaSuccess && !rt->inline_off) {
@@ -1915,11 +1933,11 @@ extern "C" int q4b_describe_dispatch(q4b_runtime *rt, int x_dtype, uint64_t m, u
         snprintf(text, text_len, "single_row_i8 one-phase persistent launch, jobs=%u (byte-addressed %u)", n_jobs, n_jobs - fast);
         return Q4B_OK;
     }
-    if (m >= 2 && m <= rt->rows_max_m && fast == n_jobs && k % 512 == 0) {
+    if (m <= rt->rows_max_m && (fast == n_jobs || m < rt->gemm_min_m)) {
         uint32_t tiles = 0, part_chunks = 0, tw = 1;
         for (const Resolved &r : resolved) tiles += (r.n + 15u) / 16u;
         const uint32_t mb = (uint32_t)(m < rt->rows_max_m ? m : rt->rows_max_m);
-        const uint32_t parts = q4k_rows_plan(mb, (uint32_t)k, tiles, (uint32_t)rt->sm_count, &part_chunks, &tw);
+        const uint32_t parts = q4k_rows_plan(mb, (uint32_t)k, tiles, (uint32_t)rt->sm_count, fast == n_jobs ? 0 : 1, &part_chunks, &tw);
         if (parts) {
             snprintf(text, text_len, "rows_i8 (short batch, integer tensor cores) rows_per_launch=%u k_parts=%u chunks_per_part=%u tiles_per_warp=%u jobs=%u (a 16-byte aligned activation is assumed)",
                      mb, parts, part_chunks, tw, n_jobs);

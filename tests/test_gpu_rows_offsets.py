@@ -1,0 +1,71 @@
+"""The short-batch kernel's byte-addressed instance: tensors at any byte offset, any whole number of affine groups, single
+rows that add to their output, and activations that are not finite. Bar: relative L2 <= 1e-5 of the 64-bit result, as for
+aligned tensors (group sums are exact integers, about 1e-7 is seen)."""
+import numpy as np
+import pytest
+
+from helpers import upload_in_one_shard, upload_matrix
+
+pytestmark = pytest.mark.gpu
+
+SEED = 20262
+
+
+@pytest.mark.parametrize("offset", [1, 2, 3, 4, 6, 8, 11, 12, 14, 15])
+@pytest.mark.parametrize("m", [2, 9])
+def test_every_offset(runtime, oracle, m, offset):
+    n, k = 75, 1536
+    trip = oracle.synth_q4(SEED, offset, n, k)
+    job = upload_matrix(runtime, *trip, offset=offset)
+    assert "rows_i8" in runtime.describe_dispatch(0, m, k, [job])
+    x = np.random.default_rng(offset).standard_normal((m, k)).astype(np.float32)
+    out = runtime.q4_affine_matmul_mapped_batch(x.reshape(-1), m, [job])[0]
+    assert oracle.rel_l2(out, oracle.matmul_f64(x, *trip, n)) <= 1e-5
+
+
+@pytest.mark.parametrize("k", [64, 128, 192, 448, 576, 1600, 5184, 17408 + 64])
+@pytest.mark.parametrize("m,offset", [(2, 0), (5, 2), (8, 13), (15, 6)])
+def test_any_number_of_groups(runtime, oracle, m, offset, k):
+    """Odd group counts leave half a last chunk, and every parameter row has a boundary of its own; the three tensors of
+    both projections lie back to back in one shard, so their offsets differ too."""
+    shapes = (33, 500)
+    trips = [oracle.synth_q4(SEED, 40 + i, n, k) for i, n in enumerate(shapes)]
+    jobs = upload_in_one_shard(runtime, trips, offset)
+    x = np.random.default_rng(k + m).standard_normal((m, k)).astype(np.float32)
+    for _ in range(2):
+        outs = runtime.q4_affine_matmul_mapped_batch(x.reshape(-1), m, jobs)
+        for out, trip, n in zip(outs, trips, shapes):
+            assert oracle.rel_l2(out, oracle.matmul_f64(x, *trip, n)) <= 1e-5
+
+
+@pytest.mark.parametrize("k,offset", [(512, 0), (704, 2), (17408, 2), (4096, 6)])
+def test_single_row_that_adds(runtime, oracle, k, offset):
+    n = 301
+    trip = oracle.synth_q4(SEED, 60, n, k)
+    job = upload_matrix(runtime, *trip, offset=offset)
+    x = np.random.default_rng(k).standard_normal((1, k)).astype(np.float32)
+    res = np.random.default_rng(k + 1).standard_normal((1, n)).astype(np.float32)
+    out = runtime.q4_affine_matmul_add_mapped_batch(x.reshape(-1), 1, [job], [res.copy()])[0]
+    assert oracle.rel_l2(out, oracle.matmul_f64(x, *trip, n) + res) <= 1e-5
+
+
+@pytest.mark.parametrize("offset", [0, 2])
+def test_outliers_and_non_finite_inputs(runtime, oracle, offset):
+    """A channel a million times the rest costs the other groups no precision; an infinity or a NaN reaches every result of
+    its own row and no other row."""
+    n, k, m = 96, 1024, 5
+    trip = oracle.synth_q4(SEED, 70, n, k)
+    x = np.random.default_rng(3).standard_normal((m, k)).astype(np.float32)
+    x[0, 100] = 1e6
+    trip[1][:, 1] = 0  # the outlier's group has scale and bias zero: what is left are the ordinary inputs
+    trip[2][:, 1] = 0
+    job = upload_matrix(runtime, *trip, offset=offset)
+    x[1] *= np.float32(1e37)
+    x[2] *= np.float32(1e-30)
+    x[3, 777] = np.inf
+    x[4, 5] = np.nan
+    out = runtime.q4_affine_matmul_mapped_batch(x.reshape(-1), m, [job])[0]
+    ref = oracle.matmul_f64(x[:3], *trip, n)
+    for r in range(3):
+        assert oracle.rel_l2(out[r], ref[r]) <= 1e-5, r
+    assert not np.isfinite(out[3:]).any()

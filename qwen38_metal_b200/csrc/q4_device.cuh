@@ -88,6 +88,10 @@ __device__ __forceinline__ uint4 lds_v4(uint32_t smem_addr) {
     return v;
 }
 
+__device__ __forceinline__ void sts_v4(uint32_t smem_addr, const uint4 &v) {
+    asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(smem_addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+
 __device__ __forceinline__ uint32_t lds_u32(uint32_t smem_addr) {
     uint32_t v;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(smem_addr) : "memory");
@@ -155,6 +159,10 @@ __device__ __forceinline__ uint32_t ldg_bf16_bits(const uint8_t *p) {
     }
     return (uint32_t)__ldg(p) | ((uint32_t)__ldg(p + 1) << 8);
 }
+
+// Device-wide fence of the hand-over "store, fence, count; count, fence, load" (__threadfence is sequentially consistent,
+// which that order does not need).
+__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
 // Programmatic dependent launch: a kernel launched with the programmatic attribute may start while the kernel before it
 // in the stream still runs. The wait returns once that kernel has finished and its writes are visible (at once when the

@@ -36,9 +36,9 @@
 // Launches are programmatic dependents of whatever runs in front of them: a block requests its first weights -- which no
 // kernel that lets a dependent start early ever writes -- and only then waits for the kernel before it.
 // What bounds it and what was measured (B200, calls back to back, before -> after the byte-addressed instance, the shared
-// B operands, the ring that does not drain and the dependent launch): 8 fp32 rows x 8192 x 5120 at a byte offset 131 -> 20.5 us
+// B operands, the ring that does not drain and the dependent launch): 8 fp32 rows x 8192 x 5120 at a byte offset 131 -> 18.9 us
 // (was: four launch pairs of the fp16 kernel), 4 rows x 34816 x 5120 35.0 -> 27.5 us (3.6 TB/s), 4 rows x 248320 x 5120 with
-// the argmax 205 -> 170 us (4.2 TB/s), one accumulating fp32 row x 5120 x 17408 at a byte offset 47.1 -> 24.9 us. Small
+// the argmax 205 -> 173 us (4.1 TB/s), one accumulating fp32 row x 5120 x 17408 at a byte offset 47.1 -> 21.5 us. Small
 // calls are bound by launch, conversion and the first round trips, long ones by the warps' instruction issue.
 #include "q4_decomp.h"
 #include "q4_device.cuh"
@@ -78,6 +78,17 @@ __host__ __device__ inline size_t rows_smem_bytes(uint32_t mp, uint32_t part_chu
 
 // Sums are carried 2^12 too small: a group's sum over 64 inputs times 0..15 of the largest fp32 numbers stays finite.
 constexpr float kRowsSumScale = 1.0f / 4096.0f;
+
+// 16 bytes starting `mis` (0..15, any value per lane) bytes into the 32-byte window {lo, hi}
+__device__ __forceinline__ uint4 realign_16_any(const uint4 &lo, const uint4 &hi, uint32_t mis) {
+    const bool by8 = (mis & 8u) != 0, by4 = (mis & 4u) != 0;
+    const uint32_t w[6] = {by8 ? lo.z : lo.x, by8 ? lo.w : lo.y, by8 ? hi.x : lo.z, by8 ? hi.y : lo.w, by8 ? hi.z : hi.x, by8 ? hi.w : hi.y};
+    uint32_t v[5];
+#pragma unroll
+    for (int i = 0; i < 5; ++i) v[i] = by4 ? w[i + 1] : w[i];
+    const uint32_t sh = (mis & 3u) * 8u;
+    return make_uint4(__funnelshift_r(v[0], v[1], sh), __funnelshift_r(v[1], v[2], sh), __funnelshift_r(v[2], v[3], sh), __funnelshift_r(v[3], v[4], sh));
+}
 
 // exponent that puts a group's largest magnitude into [2^21, 2^22); both 2^e and 2^-e are normal numbers. Magnitudes
 // below 2^-105 keep an absolute step of 2^-126.
@@ -171,15 +182,24 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
         if (pc != pc_stop) {
             const uint32_t stage = ring + req_stage * kStage;
             const bool in = !MIS || pc < pc_end;
-            const bool has_b = !MIS || 2u * pc + 1u < p.groups;
+            if (!MIS || (in && 2u * pc + 1u < p.groups)) {
+#pragma unroll
+                for (int w = 0; w < TW; ++w) {
+                    cp_async_16(stage + w * kRowsStageBytes + copy_off, wa[w]);
+                    cp_async_16(stage + w * kRowsStageBytes + 512u + copy_off, wb[w]);
+                }
+            } else {
+                // at the end of a row or run only windows that hold bytes of the row (q4_decomp.h); the stage after the run's
+                // last chunk holds the window that completes that chunk
+#pragma unroll
+                for (int w = 0; w < TW; ++w) {
+                    const bool pred = in ? q4_window_wanted(cq, wmis[w], false) : pc == pc_end && cq == 0 && q4_fifth_window_wanted(wmis[w], 2u * pc - 1u < p.groups);
+                    cp_async_16_pred(stage + w * kRowsStageBytes + copy_off, wa[w], pred);
+                    cp_async_16_pred(stage + w * kRowsStageBytes + 512u + copy_off, wb[w], pred);
+                }
+            }
 #pragma unroll
             for (int w = 0; w < TW; ++w) {
-                // only windows that hold bytes of the row (q4_decomp.h); the stage after the run's last chunk holds the
-                // window that completes that chunk
-                bool pred = true;
-                if (MIS) pred = in ? q4_window_wanted(cq, wmis[w], has_b) : pc == pc_end && cq == 0 && q4_fifth_window_wanted(wmis[w], 2u * pc - 1u < p.groups);
-                cp_async_16_pred(stage + w * kRowsStageBytes + copy_off, wa[w], pred);
-                cp_async_16_pred(stage + w * kRowsStageBytes + 512u + copy_off, wb[w], pred);
                 wa[w] += 64;
                 wb[w] += 64;
             }
@@ -188,7 +208,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
 #pragma unroll
                 for (int w = 0; w < TW; ++w) {
                     const uint32_t dst = pring + req_param * kParamStage + w * kParamTile + lane * 16u;
-                    cp_async_16_pred(dst, pw[w], true);
+                    cp_async_16(dst, pw[w]);
                     if (MIS) cp_async_16_pred(dst + 512u, pw[w] + 16, pown[w] + 2u * min(8u, p.groups - 2u * pc) > 16u);
                     pw[w] += 16;
                 }
@@ -326,7 +346,9 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
         const uint32_t c_begin = c_lo + 4u * q0, c_stop = min(c_lo + 4u * q1, c_hi);
         u += q1 - q0;
         const RowsJob *job[TW];
-        uint32_t row0[TW], wm[TW], pmis[TW];  // pmis: parameter rows g, g + 8 of the scales and of the biases, four bits each
+        uint32_t row0[TW], wm[TW], pmis[TW];  // pmis: of the parameter row this lane copied (and realigns)
+        uint32_t rlo[TW][2], rhi[TW][2];      // where this lane's two 8-byte words of each group are in a stage ...
+        bool nlo[TW], nhi[TW];                // ... and whether those of the second group are in the next stage
         bool tile_live[TW];
 #pragma unroll
         for (int w = 0; w < TW; ++w) {
@@ -334,10 +356,15 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
             wm[w] = pmis[w] = 0;
             if (MIS) {
                 wm[w] = (uint32_t)((uintptr_t)job[w]->w & 15u);
-                const uint32_t last = job[w]->n - 1u, ra = min(row0[w] + g, last), rb = min(row0[w] + 8u + g, last);
-                const uint32_t ps = (uint32_t)(uintptr_t)job[w]->s, pb = (uint32_t)(uintptr_t)job[w]->b;  // (runs begin at multiples of 16 bytes)
-                pmis[w] = ((ps + ra * p.groups * 2u) & 15u) | ((ps + rb * p.groups * 2u) & 15u) << 4 | ((pb + ra * p.groups * 2u) & 15u) << 8 |
-                          ((pb + rb * p.groups * 2u) & 15u) << 12;
+                const uint32_t j = t + (wm[w] >> 3);
+                rlo[w][0] = word_off(j);
+                rhi[w][0] = word_off(j + 1u);
+                rlo[w][1] = word_off(j + 4u);
+                rhi[w][1] = word_off(j + 5u);
+                nlo[w] = j + 4u >= 8u;
+                nhi[w] = j + 5u >= 8u;
+                const uint32_t rp = min(row0[w] + (lane & 15u), job[w]->n - 1u);
+                pmis[w] = ((uint32_t)(uintptr_t)((lane >> 4) ? job[w]->b : job[w]->s) + rp * p.groups * 2u) & 15u;  // (runs begin at multiples of 16 bytes)
             }
         }
         float acc[TW][NB][AV];
@@ -351,22 +378,28 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
             const uint32_t pst = pring + param_i * kParamStage;
             const uint32_t xc = xdig_addr + (c - c_lo) * rows_chunk_bytes(MP);
             const uint32_t xs = xscale_addr + (c - c_lo) * (2u * MP * rows_scale_bytes(DC));
+            if (MIS && (c & 3u) == 0) {
+                // a new quad: lane l shifts the parameter row it copied to the boundary, groups past the last one become zero
+                const uint32_t left = p.groups - 2u * c;
+#pragma unroll
+                for (int w = 0; w < TW; ++w) {
+                    const uint32_t at = pst + w * kParamTile + lane * 16u;
+                    uint4 v = realign_16_any(lds_v4(at), lds_v4(at + 512u), pmis[w]);
+                    if (left < 8u) {
+                        uint32_t *r = &v.x;
+#pragma unroll
+                        for (uint32_t i = 0; i < 4u; ++i) r[i] = 2u * i >= left ? 0u : 2u * i + 1u >= left ? r[i] & 0xffffu : r[i];
+                    }
+                    sts_v4(at, v);
+                }
+                __syncwarp();
+            }
             // scales and biases of the chunk's two groups, rows g and g + 8
             uint32_t prm[TW][4];
 #pragma unroll
             for (int w = 0; w < TW; ++w)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const uint32_t at = pst + w * kParamTile + (i >> 1) * 256u + (g + 8u * (i & 1)) * 16u, byte = (c & 3u) * 4u;
-                    if (!MIS) {
-                        prm[w][i] = lds_u32(at + byte);
-                    } else {
-                        const uint32_t o = ((pmis[w] >> (4 * i)) & 15u) + byte, w0 = o >> 2, w1 = w0 + 1u;
-                        const uint32_t lo = lds_u32(at + (w0 & 4u) * 128u + (w0 & 3u) * 4u), hi = lds_u32(at + (w1 & 4u) * 128u + (w1 & 3u) * 4u);
-                        prm[w][i] = __funnelshift_r(lo, hi, (o & 3u) * 8u);
-                        if (2u * c + 1u >= p.groups) prm[w][i] &= 0xffffu;  // no second group in the last chunk
-                    }
-                }
+                for (int i = 0; i < 4; ++i) prm[w][i] = lds_u32(pst + w * kParamTile + (i >> 1) * 256u + (g + 8u * (i & 1)) * 16u + (c & 3u) * 4u);
 #pragma unroll
             for (int grp = 0; grp < 2; ++grp) {
                 // the activation's digits of this group: read once, used by every tile of the item
@@ -391,8 +424,8 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
                         wA = lds_v2(wst + (grp ? rd1 : rd0));
                         wB = lds_v2(wst + 512u + (grp ? rd1 : rd0));
                     } else {
-                        const uint32_t j0 = 4u * grp + t + (wm[w] >> 3), j1 = j0 + 1u, nst = next_stage + w * kRowsStageBytes;
-                        const uint32_t a0 = (j0 < 8u ? wst : nst) + word_off(j0), a1 = (j1 < 8u ? wst : nst) + word_off(j1);
+                        const uint32_t nst = next_stage + w * kRowsStageBytes;
+                        const uint32_t a0 = (grp && nlo[w] ? nst : wst) + rlo[w][grp], a1 = (grp && nhi[w] ? nst : wst) + rhi[w][grp];
                         const uint2 loA = lds_v2(a0), hiA = lds_v2(a1), loB = lds_v2(a0 + 512u), hiB = lds_v2(a1 + 512u);
                         const uint32_t sh = (wm[w] & 3u) * 8u;
                         const bool by4 = (wm[w] & 4u) != 0;
@@ -478,7 +511,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
 #pragma unroll
                     for (int i = 0; i < AV; ++i)
                         if (mine) p.partials[(slot * MP + act_row(nb, i)) * rows_total + (size_t)(item * TW + w) * 16u + weight_row(i)] = acc[w][nb][i];
-            __threadfence();
+            fence_gpu();
             __syncwarp();
             unsigned int before = 0;
             if (lane == 0) before = atomicAdd(p.counters + item, 1u);
@@ -489,27 +522,37 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
             before = __shfl_sync(0xffffffffu, before, 0);
             last = before + 1u == __reduce_add_sync(0xffffffffu, shares);
             if (last) {
-                __threadfence();
+                fence_gpu();
                 if (lane == 0) p.counters[item] = 0;  // ready for the next launch
             }
         }
         if (last) {
             if (!whole) {
-                // all contributions in K order, whoever came last
+                // all contributions in K order, whoever came last; four at a time, so that a round trip to L2 fetches four
 #pragma unroll
                 for (int i = 0; i < TW * NB * AV; ++i) (&acc[0][0][0])[i] = 0.f;
-                for (uint32_t pp = 0; pp < p.parts; ++pp) {
-                    const uint32_t n = __shfl_sync(0xffffffffu, shares, pp);
-                    for (uint32_t j = 0; j < n; ++j) {
-                        const float *src = p.partials + ((size_t)pp * p.part_slots + j) * MP * rows_total;
+                uint32_t pp = 0, jj = 0, n = __shfl_sync(0xffffffffu, shares, 0);
+                while (pp < p.parts) {
+                    constexpr int B = 4;
+                    float got[B][TW * NB * AV];
 #pragma unroll
-                        for (int w = 0; w < TW; ++w)
+                    for (int b = 0; b < B; ++b) {
+                        const bool have = pp < p.parts;  // (uniform)
+                        const float *src = p.partials + ((size_t)pp * p.part_slots + jj) * MP * rows_total + (size_t)item * TW * 16u;
 #pragma unroll
-                            for (int nb = 0; nb < NB; ++nb)
-#pragma unroll
-                                for (int i = 0; i < AV; ++i)
-                                    acc[w][nb][i] += __ldcg(src + (size_t)act_row(nb, i) * rows_total + (size_t)(item * TW + w) * 16u + weight_row(i));
+                        for (int v = 0; v < TW * NB * AV; ++v) {
+                            const int i = v % AV, nb = v / AV % NB, w = v / (AV * NB);
+                            got[b][v] = have ? __ldcg(src + (size_t)act_row(nb, i) * rows_total + w * 16u + weight_row(i)) : 0.f;
+                        }
+                        if (have && ++jj == n) {
+                            jj = 0;
+                            n = __shfl_sync(0xffffffffu, shares, ++pp & 31u);
+                        }
                     }
+#pragma unroll
+                    for (int b = 0; b < B; ++b)
+#pragma unroll
+                        for (int v = 0; v < TW * NB * AV; ++v) (&acc[0][0][0])[v] += got[b][v];
                 }
             }
 #pragma unroll

@@ -75,14 +75,13 @@ struct RowsParams {
     uint32_t k, groups, cpt;  // inputs, k / 64, chunks of 128 inputs (the last may hold one group)
     uint32_t parts;        // runs the K range is cut into (q4k_rows_plan)
     uint32_t part_chunks;  // chunks of the longest run
-    uint32_t tiles_per_warp;  // 1, or 2 (up to 8 rows): two tiles share the activation's fragments
     uint32_t tiles;        // 16-row tiles of all jobs
     uint32_t run;          // quads of chunks per warp (q4_rows_run)
     uint32_t part_slots;   // most contributions a part makes to one tile (q4_rows_part_slots)
     uint32_t accumulate;
     uint32_t byte_addressed;  // some tensor misses a 16-byte boundary, or K % 512 != 0
-    float *partials;       // [parts][part_slots][padded rows][items * tiles_per_warp * 16] fp32, for tiles with several contributions
-    unsigned int *counters;  // [items], zero between launches
+    float *partials;       // [parts][part_slots][padded rows][tiles * 16] fp32, for tiles with several contributions
+    unsigned int *counters;  // [tiles], zero between launches
     unsigned long long *trace;  // optional [warps of the grid][4] globaltimer stamps (start, digits ready, first tile streamed, done)
 };
 
@@ -101,7 +100,7 @@ cudaError_t q4k_prepare_x(const void *x, int x_is_f32, uint32_t m_rows, uint32_t
 cudaError_t q4k_gemv(const q4::GemvParams *params, int column_tiles, int aligned, cudaStream_t stream);  // one warp per block
 uint32_t q4k_gemv_occupancy(int column_tiles, int aligned);  // resident warps per SM, 0 on error
 
-uint32_t q4k_rows_plan(uint32_t m, uint32_t k, uint32_t tiles, uint32_t sm_count, int mis, uint32_t *part_chunks, uint32_t *tiles_per_warp);  // parts, 0: unsupported
+uint32_t q4k_rows_plan(uint32_t m, uint32_t k, uint32_t tiles, uint32_t sm_count, int mis, uint32_t *part_chunks);  // parts, 0: unsupported
 uint32_t q4k_rows_padded(uint32_t m);  // activation rows a launch of m rows holds
 cudaError_t q4k_rows(const q4::RowsParams *params, uint32_t sm_count, cudaStream_t stream);
 

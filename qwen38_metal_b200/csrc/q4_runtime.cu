@@ -487,8 +487,8 @@ int launch_rows(q4b_runtime *rt, const void *x_dev, int x_dtype, uint32_t m, uin
     uint32_t tiles = 0;
     for (uint32_t i = 0; i < n_jobs; ++i) tiles += (jobs[i].n + 15u) / 16u;
     const int mis = rows_byte_addressed(jobs, n_jobs, k / 64u) ? 1 : 0;
-    uint32_t part_chunks = 0, tiles_per_warp = 1;
-    const uint32_t parts = q4k_rows_plan(m, k, tiles, (uint32_t)rt->sm_count, mis, &part_chunks, &tiles_per_warp);
+    uint32_t part_chunks = 0;
+    const uint32_t parts = q4k_rows_plan(m, k, tiles, (uint32_t)rt->sm_count, mis, &part_chunks);
     if (parts == 0) return -1;
     q4::RowsParams p;
     memset(&p, 0, sizeof p);
@@ -517,16 +517,14 @@ int launch_rows(q4b_runtime *rt, const void *x_dev, int x_dtype, uint32_t m, uin
     p.byte_addressed = (uint32_t)mis;
     p.parts = parts;
     p.part_chunks = part_chunks;
-    p.tiles_per_warp = tiles_per_warp;
     p.tiles = tiles;
     p.accumulate = (flags & Q4B_FLAG_ACCUMULATE) ? 1u : 0u;
-    const uint32_t items = (tiles + tiles_per_warp - 1u) / tiles_per_warp;
-    p.run = q4_rows_run(items, part_chunks, parts, (uint32_t)rt->sm_count);
+    p.run = q4_rows_run(tiles, part_chunks, parts, (uint32_t)rt->sm_count);
     p.part_slots = q4_rows_part_slots(p.cpt, parts, p.run);
     if (parts > 1 || p.part_slots > 1) {
-        Q4B_CUDA(rt->rows_partials.ensure((size_t)parts * p.part_slots * q4k_rows_padded(m) * items * tiles_per_warp * 16 * 4), "partial sum scratch");
+        Q4B_CUDA(rt->rows_partials.ensure((size_t)parts * p.part_slots * q4k_rows_padded(m) * tiles * 16 * 4), "partial sum scratch");
         const size_t had = rt->rows_counters.capacity;
-        Q4B_CUDA(rt->rows_counters.ensure((size_t)items * 4), "tile counter scratch");
+        Q4B_CUDA(rt->rows_counters.ensure((size_t)tiles * 4), "tile counter scratch");
         // the counters are put back to zero by the kernel itself; after a failed command on this runtime (a launch may
         // have been cut short) and for a fresh buffer they are cleared here
         if (rt->rows_counters.capacity != had || rt->rows_failures_seen != rt->failures) {
@@ -560,7 +558,7 @@ int enqueue_matmul(q4b_runtime *rt, const void *x_dev, int x_dtype, uint64_t m, 
     bool rows = !want_tensor && (m >= 2 || (!single && m < rt->gemm_min_m)) && rt->rows_max_m >= 2 && (want_stream || m <= rt->rows_max_m) &&
                 ((uintptr_t)x_dev & 15u) == 0;
     for (size_t j0 = 0; j0 < jobs.size() && rows; j0 += q4::kMaxJobs) {
-        uint32_t tiles = 0, part_chunks = 0, tw = 1;
+        uint32_t tiles = 0, part_chunks = 0;
         const uint32_t nj = (uint32_t)std::min(jobs.size() - j0, (size_t)q4::kMaxJobs);
         for (size_t j = j0; j < j0 + nj; ++j) tiles += (jobs[j].n + 15u) / 16u;
         const int mis = rows_byte_addressed(&jobs[j0], nj, (uint32_t)(k / 64)) ? 1 : 0;
@@ -569,8 +567,8 @@ int enqueue_matmul(q4b_runtime *rt, const void *x_dev, int x_dtype, uint64_t m, 
             rows = false;
             break;
         }
-        rows = q4k_rows_plan(full, (uint32_t)k, tiles, (uint32_t)rt->sm_count, mis, &part_chunks, &tw) != 0 &&
-               (m <= rt->rows_max_m || rest == 0 || q4k_rows_plan(rest, (uint32_t)k, tiles, (uint32_t)rt->sm_count, mis, &part_chunks, &tw) != 0);
+        rows = q4k_rows_plan(full, (uint32_t)k, tiles, (uint32_t)rt->sm_count, mis, &part_chunks) != 0 &&
+               (m <= rt->rows_max_m || rest == 0 || q4k_rows_plan(rest, (uint32_t)k, tiles, (uint32_t)rt->sm_count, mis, &part_chunks) != 0);
     }
     if (rows) {
         for (uint64_t m0 = 0; m0 < m; m0 += rt->rows_max_m) {
@@ -1934,13 +1932,13 @@ extern "C" int q4b_describe_dispatch(q4b_runtime *rt, int x_dtype, uint64_t m, u
         return Q4B_OK;
     }
     if (m <= rt->rows_max_m && (fast == n_jobs || m < rt->gemm_min_m)) {
-        uint32_t tiles = 0, part_chunks = 0, tw = 1;
+        uint32_t tiles = 0, part_chunks = 0;
         for (const Resolved &r : resolved) tiles += (r.n + 15u) / 16u;
         const uint32_t mb = (uint32_t)(m < rt->rows_max_m ? m : rt->rows_max_m);
-        const uint32_t parts = q4k_rows_plan(mb, (uint32_t)k, tiles, (uint32_t)rt->sm_count, fast == n_jobs ? 0 : 1, &part_chunks, &tw);
+        const uint32_t parts = q4k_rows_plan(mb, (uint32_t)k, tiles, (uint32_t)rt->sm_count, fast == n_jobs ? 0 : 1, &part_chunks);
         if (parts) {
-            snprintf(text, text_len, "rows_i8 (short batch, integer tensor cores) rows_per_launch=%u k_parts=%u chunks_per_part=%u tiles_per_warp=%u jobs=%u (a 16-byte aligned activation is assumed)",
-                     mb, parts, part_chunks, tw, n_jobs);
+            snprintf(text, text_len, "rows_i8 (short batch, integer tensor cores) rows_per_launch=%u k_parts=%u chunks_per_part=%u jobs=%u (a 16-byte aligned activation is assumed)",
+                     mb, parts, part_chunks, n_jobs);
             return Q4B_OK;
         }
     }

@@ -524,7 +524,7 @@ def run_ours(args) -> int:
             "path": ("persistent decode chain (one cooperative launch per token and GPU"
                      + (", peer stores + cross-GPU barriers)" if world > 1 else ")")) if chain is not None
                     else "CUDA graph of per-stage launches + NCCL all-gathers",
-            "roofline": {"bound": "hbm", "kernel": "q4_stack_inline_kernel (per-stage launches, one per projection group)", "achieved": achieved, "peak": peak,
+            "roofline": {"bound": "hbm", "kernel": "q4_rows_kernel (per-stage launches, one per projection group; a byte-addressed lm_head: q4_stack_inline_kernel)", "achieved": achieved, "peak": peak,
                          "peak_source": peak_source, "unit": UNIT, "frac": achieved / peak if peak else None,
                          "frac_of_8TBs": achieved / NOMINAL_HBM_GBS, "launches": prof["launches"],
                          "avg_launch_us": prof["ms"] * 1e3 / max(1, prof["launches"]),

@@ -36,11 +36,12 @@
 // Launches are programmatic dependents of whatever runs in front of them: a block requests its first weights -- which no
 // kernel that lets a dependent start early ever writes -- and only then waits for the kernel before it.
 // What bounds it and what was measured (B200, a graph of calls, one call; in brackets the ring of single chunks with a rolled
-// loop, which issued 162 warp instructions a chunk where 100 will do): 4 rows x 34816 x 5120 24.9 us = 4.0 TB/s (26.0), 4 rows x
-// 248320 x 5120 129 us = 5.5 TB/s (147), 8 fp32 rows x 8192 x 5120 at a byte offset 17.0 us (18.5), one fp32 row x 5120 x 17408 at a
-// byte offset 18.4 us (20.1), 16 rows x 34816 x 5120 63 us (67). Eight rows x 34816 x 5120 take 31.1 us; a form that walked two
+// loop, which issued 162 warp instructions a chunk where 100 will do): 4 rows x 34816 x 5120 24.3 us = 4.1 TB/s (26.0), 4 rows x
+// 248320 x 5120 129 us = 5.5 TB/s (147), 8 fp32 rows x 8192 x 5120 at a byte offset 16.3 us (18.5), one fp32 row x 5120 x 17408 at a
+// byte offset 16.6 us (20.1), 16 rows x 34816 x 5120 63 us (67). Eight rows x 34816 x 5120 take 31.1 us; a form that walked two
 // tiles at a time took 28.8 there and lost everywhere else. Small calls are bound by launch, conversion and the first round
 // trips (2.5 us until the digits are ready, 2 us for the contributions to meet), long ones by the warps' instruction issue.
+// Requesting the second half of the ring only after the activation is out costs 0.6 us in a row of calls and gains nothing.
 #include "q4_decomp.h"
 #include "q4_device.cuh"
 #include "q4_kernels.h"
@@ -52,13 +53,13 @@ constexpr int kRowsStageBytes = 1024;  // one chunk of one tile: 16 weight rows 
 constexpr int kRowsPerThread = 8;      // blocks of 8 inputs a thread converts at most (bounds a part: rows x chunks <= 256)
 constexpr uint32_t kRowsPairColumns = 4;  // up to this many rows share B operands in pairs
 
-// A warp's ring has two halves of a quad each: four 1 KB chunks of one tile, the scales and biases of their eight groups (a
-// 16-byte window per row and array; two of them when they may start anywhere) and, byte-addressed, the window that
-// completes the fourth chunk of every row. One half is consumed while the other one is on its way; the loop over a
-// quad is unrolled, so that every address in it is a constant from the half's base.
-__host__ __device__ constexpr uint32_t rows_tail_bytes(bool mis) { return mis ? 256u : 0u; }
-__host__ __device__ constexpr uint32_t rows_param_bytes(bool mis) { return mis ? 1024u : 512u; }
-__host__ __device__ constexpr uint32_t rows_half_bytes(bool mis) { return 4u * kRowsStageBytes + rows_tail_bytes(mis) + rows_param_bytes(mis); }
+// A warp's ring has two halves of a quad each: four 1 KB chunks of one tile and the scales and biases of their eight groups
+// (a 16-byte window per row and array). Byte-addressed, a fifth stage follows the four: the first quarter of its rows
+// holds the window that completes the fourth chunk, where a following chunk would have it, and the second and third
+// quarters the second windows of the parameters. One half is consumed while the other one is on its way; the loop
+// over a quad is unrolled, so that every address in it is a constant from the half's base.
+__host__ __device__ constexpr uint32_t rows_weight_bytes(bool mis) { return (mis ? 5u : 4u) * kRowsStageBytes; }
+__host__ __device__ constexpr uint32_t rows_half_bytes(bool mis) { return rows_weight_bytes(mis) + 512u; }
 
 __host__ __device__ constexpr bool rows_dc(uint32_t m) { return m <= kRowsPairColumns; }
 __host__ __device__ constexpr uint32_t rows_padded(uint32_t m) { return rows_dc(m) ? (m + 1u) & ~1u : (m + 7u) & ~7u; }
@@ -99,11 +100,16 @@ __device__ __forceinline__ unsigned long long rows_ns() {
     return t;
 }
 
+template <int F>
+struct Form {
+    static constexpr int value = F;
+};
+
 template <int NB, bool DC, bool MIS>
 __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __grid_constant__ RowsParams p) {
     constexpr uint32_t MP = (DC ? 2 : 8) * NB;
     constexpr uint32_t T = kRowsWarps * 32;
-    constexpr uint32_t kHalf = rows_half_bytes(MIS), kTail = 4u * kRowsStageBytes, kParams = kTail + rows_tail_bytes(MIS);
+    constexpr uint32_t kHalf = rows_half_bytes(MIS), kTail = 4u * kRowsStageBytes, kParams = rows_weight_bytes(MIS);
     extern __shared__ __align__(128) uint8_t smem[];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t g = lane >> 2, t = lane & 3u;
@@ -118,6 +124,8 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
     // that the 8-byte reads below (lane (g, t): bytes 8 t.. of a group) touch every bank once per half-warp.
     const uint32_t cr = lane >> 2, cq = lane & 3u;
     const uint32_t copy_off = 16u * (cr * 4u + (cq ^ (2u * ((cr >> 1) & 1u))));
+    // second window of the parameter row that lane l copies: row l & 15 of the fifth stage, quarter 1 (scales) or 2 (biases)
+    const uint32_t second_off = kTail + 64u * (lane & 15u) + 16u * ((1u + (lane >> 4)) ^ (2u * ((lane >> 1) & 1u)));
     const uint64_t row_bytes = (uint64_t)p.k >> 1;
     const uint32_t quads = (nch + 3u) / 4u;
     const uint32_t worker = gi * kRowsWarps + warp;
@@ -166,24 +174,24 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
                 }
                 if (MIS) {
                     const bool pred = cq == 0 && q4_fifth_window_wanted(wmis, true);
-                    cp_async_16_pred(base + kTail + cr * 16u, wa + 256, pred);
-                    cp_async_16_pred(base + kTail + 128u + cr * 16u, wb + 256, pred);
+                    cp_async_16_pred(base + kTail + copy_off, wa + 256, pred);
+                    cp_async_16_pred(base + kTail + 512u + copy_off, wb + 256, pred);
                 }
             } else {
-                // at the end of a row only windows that hold bytes of the row (q4_decomp.h); the stage after the last chunk (or
-                // the tail) holds the window that completes that chunk
+                // at the end of a row only windows that hold bytes of the row (q4_decomp.h); the stage after the last chunk holds
+                // the window that completes it
 #pragma unroll
                 for (int s = 0; s < 5; ++s) {
                     const uint32_t c = pc + s;
                     const bool fifth = cq == 0 && c == pc_end && q4_fifth_window_wanted(wmis, 2u * c - 1u < p.groups);
                     const bool pred = (s < 4 && c < pc_end) ? q4_window_wanted(cq, wmis, 2u * c + 1u < p.groups) : fifth;
-                    cp_async_16_pred(s < 4 ? base + s * kRowsStageBytes + copy_off : base + kTail + cr * 16u, wa + s * 64, pred);
-                    cp_async_16_pred(s < 4 ? base + s * kRowsStageBytes + 512u + copy_off : base + kTail + 128u + cr * 16u, wb + s * 64, pred);
+                    cp_async_16_pred(base + s * kRowsStageBytes + copy_off, wa + s * 64, pred);
+                    cp_async_16_pred(base + s * kRowsStageBytes + 512u + copy_off, wb + s * 64, pred);
                 }
             }
             // lane l copies the scales (l < 16) or biases of row l & 15 for the quad's eight groups
             cp_async_16(base + kParams + lane * 16u, pw);
-            if (MIS) cp_async_16_pred(base + kParams + 512u + lane * 16u, pw + 16, pown + 2u * min(8u, p.groups - 2u * pc) > 16u);
+            if (MIS) cp_async_16_pred(base + second_off, pw + 16, pown + 2u * min(8u, p.groups - 2u * pc) > 16u);
             wa += 256;
             wb += 256;
             pw += 16;
@@ -206,7 +214,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
     // flight at once: one round trip to L2 instead of one per block.
     const uint32_t span8 = nch * 16u;  // blocks of 8 inputs per row in this part
     uint4 raw[kRowsPerThread][2];
-    const uint32_t total8 = p.m * span8, padded8 = MP * span8;  // rows past m are zero-filled
+    const uint32_t total8 = p.m * span8, todo8 = DC ? total8 : MP * span8;  // rows past m: zeros (DC: their columns stay zero)
 #pragma unroll
     for (int i = 0; i < kRowsPerThread; ++i) {
         const uint32_t idx = threadIdx.x + i * T;
@@ -253,9 +261,9 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
     // the eight threads of a group agree on its scale (span8 is a multiple of 16: a group never leaves its half-warp)
 #pragma unroll
     for (int i = 0; i < kRowsPerThread; ++i) {
-        if ((uint32_t)i * T >= padded8) continue;  // (uniform)
+        if ((uint32_t)i * T >= todo8) continue;  // (uniform)
         const uint32_t idx = threadIdx.x + i * T;
-        const bool live = idx < padded8;
+        const bool live = idx < todo8;
         const uint32_t mrow = live ? idx / span8 : 0u, b8 = live ? idx - mrow * span8 : 0u;
         float v[8];
         unpack8(raw[i], v);
@@ -298,8 +306,8 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
 
     // ---- tiles ----
     // B operands: digit d of row g of a block of eight (16 bytes from lane t); DC: digit g & 3 of row g >> 2 of a pair, zeros
-    // in columns 3 and 7
-    const bool has_x = !DC || (g & 3u) < 3u;
+    // in columns 3 and 7 and in those of a row past m
+    auto has_x = [&](int nb) { return (g & 3u) < 3u && nb * 2u + (g >> 2) < p.m; };
     const uint32_t xdig_addr = (uint32_t)__cvta_generic_to_shared(xdig) + (DC ? (g >> 2) * 192u + (g & 3u) * 64u : g * 64u) + t * 16u;
     const uint32_t xscale_addr = (uint32_t)__cvta_generic_to_shared(xscale) + (DC ? (t >> 1) * 16u + (t & 1u) * 8u : t * 16u);
     constexpr int XD = DC ? 1 : 3;  // B operands of a group and block of rows
@@ -307,9 +315,9 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
 #pragma unroll
     for (int i = 0; i < 2 * NB * XD; ++i) (&xf[0][0][0])[i] = make_uint4(0, 0, 0, 0);
     // this lane's 8 bytes of group G of row g in a stage: word j = 4 G + t of the row's eight 8-byte words, in quarter
-    // j >> 1, swizzled as above; words 8 and 9 (MIS) are the first two of the next stage, or of the tail
+    // j >> 1, swizzled as above; words 8 and 9 (MIS) are the first two of the next stage
     const uint32_t rd_swz = 2u * ((g >> 1) & 1u);
-    auto word_off = [&](uint32_t j) { return 16u * (g * 4u + (((j >> 1) & 3u) ^ rd_swz)) + 8u * (j & 1u); };
+    auto word_off = [&](uint32_t j) { return (j >> 3) * kRowsStageBytes + 16u * (g * 4u + (((j >> 1) & 3u) ^ rd_swz)) + 8u * (j & 1u); };
     const uint32_t rd0 = word_off(t), rd1 = word_off(4u + t);
     constexpr int AV = DC ? 2 : 4;  // sums a lane holds per tile and block of rows
     uint32_t half = 0;
@@ -321,8 +329,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
         uint32_t row0;
         find_tile(tile, job, row0);
         uint32_t wm = 0, pmis = 0;  // pmis: of the parameter row this lane copied (and realigns)
-        uint32_t rlo[2], rhi[2];    // where this lane's two 8-byte words of each group are in a stage ...
-        bool nlo = false, nhi = false;  // ... and whether those of the second group are in the next one
+        uint32_t rlo[2] = {0, 0}, rhi[2] = {0, 0};  // where this lane's two 8-byte words of each group are, from a chunk's stage
         if (MIS) {
             wm = (uint32_t)((uintptr_t)job->w & 15u);
             const uint32_t j = t + (wm >> 3);
@@ -330,8 +337,6 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
             rhi[0] = word_off(j + 1u);
             rlo[1] = word_off(j + 4u);
             rhi[1] = word_off(j + 5u);
-            nlo = j + 4u >= 8u;
-            nhi = j + 5u >= 8u;
             const uint32_t rp = min(row0 + (lane & 15u), job->n - 1u);
             pmis = ((uint32_t)(uintptr_t)((lane >> 4) ? job->b : job->s) + rp * p.groups * 2u) & 15u;  // (runs begin at multiples of 16 bytes)
         }
@@ -347,7 +352,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
             if (MIS) {
                 // lane l shifts the parameter row it copied to the boundary, groups past the last one become zero
                 const uint32_t left = p.groups - 2u * c;
-                uint4 v = realign_16_any(lds_v4(pst + lane * 16u), lds_v4(pst + 512u + lane * 16u), pmis);
+                uint4 v = realign_16_any(lds_v4(pst + lane * 16u), lds_v4(base + second_off), pmis);
                 if (left < 8u) {
                     uint32_t *r = &v.x;
 #pragma unroll
@@ -360,9 +365,11 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
             uint4 prm[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) prm[i] = lds_v4(pst + (i >> 1) * 256u + (g + 8u * (i & 1)) * 16u);
-#pragma unroll
-            for (int s = 0; s < 4; ++s) {
-                if (MIS && c + s >= c_stop) break;  // (uniform)
+            // One chunk. `form`: the weights are aligned (0), miss a boundary by less than four bytes of every eight (1) or by four
+            // or more (2), or whatever wm says (3): a branch inside the chunk would keep the loads of one group from
+            // overlapping the arithmetic of the one before it (one row x 248320 x 5120 at a byte offset: 164 -> 151 us).
+            auto chunk = [&](auto form, int s) {
+                constexpr int F = decltype(form)::value;
                 const uint32_t stage = base + s * kRowsStageBytes;
                 uint32_t pr[4];
 #pragma unroll
@@ -374,7 +381,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
                     for (int nb = 0; nb < NB; ++nb) {
                         const uint32_t xcs = xc + s * rows_chunk_bytes(MP), xss = xs + s * (2u * MP * rows_scale_bytes(DC));
                         if constexpr (DC) {
-                            lds_v4_keep(xf[grp][nb][0], xcs + (uint32_t)(grp * 3 * MP * 64 + nb * 384), has_x);
+                            lds_v4_keep(xf[grp][nb][0], xcs + (uint32_t)(grp * 3 * MP * 64 + nb * 384), has_x(nb));
                             const uint2 f = lds_v2(xss + (uint32_t)((grp * MP + nb * 2) * 16));
                             xv[nb] = make_uint4(f.x, f.y, 0, 0);
                         } else {
@@ -384,23 +391,34 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
                         }
                     }
                     uint2 wA, wB;
-                    if (!MIS || wm == 0) {
+                    if (F == 0 || (F == 3 && wm == 0)) {
                         wA = lds_v2(stage + (grp ? rd1 : rd0));
                         wB = lds_v2(stage + 512u + (grp ? rd1 : rd0));
                     } else {
-                        // (words past the stage: the next stage keeps its rows 64 bytes apart, the tail 16)
-                        const uint32_t past = s < 3 ? stage + kRowsStageBytes + g * 64u + rd_swz * 16u : base + kTail + g * 16u, past_b = s < 3 ? 512u : 128u;
-                        const bool lo_past = grp && nlo, hi_past = grp && nhi;
-                        const uint32_t odd = 8u * ((t + (wm >> 3)) & 1u);
-                        const uint32_t a0 = lo_past ? past + odd : stage + rlo[grp], a1 = hi_past ? past + (odd ^ 8u) : stage + rhi[grp];
-                        const uint2 loA = lds_v2(a0), hiA = lds_v2(a1);
-                        const uint2 loB = lds_v2(a0 + (lo_past ? past_b : 512u)), hiB = lds_v2(a1 + (hi_past ? past_b : 512u));
-                        const uint32_t sh = (wm & 3u) * 8u;
-                        const bool by4 = (wm & 4u) != 0;
-                        wA.x = __funnelshift_r(by4 ? loA.y : loA.x, by4 ? hiA.x : loA.y, sh);
-                        wA.y = __funnelshift_r(by4 ? hiA.x : loA.y, by4 ? hiA.y : hiA.x, sh);
-                        wB.x = __funnelshift_r(by4 ? loB.y : loB.x, by4 ? hiB.x : loB.y, sh);
-                        wB.y = __funnelshift_r(by4 ? hiB.x : loB.y, by4 ? hiB.y : hiB.x, sh);
+                        // the word the lane's bytes begin in and the two after it: a 64-bit and a 32-bit read
+                        const uint32_t a0 = stage + rlo[grp], a1 = stage + rhi[grp], sh = (wm & 3u) * 8u;
+                        uint32_t va[3], vb[3];
+                        if (F == 2 || (F == 3 && (wm & 4u))) {
+                            const uint2 hiA = lds_v2(a1), hiB = lds_v2(a1 + 512u);
+                            va[0] = lds_u32(a0 + 4u);
+                            vb[0] = lds_u32(a0 + 516u);
+                            va[1] = hiA.x;
+                            va[2] = hiA.y;
+                            vb[1] = hiB.x;
+                            vb[2] = hiB.y;
+                        } else {
+                            const uint2 loA = lds_v2(a0), loB = lds_v2(a0 + 512u);
+                            va[2] = lds_u32(a1);
+                            vb[2] = lds_u32(a1 + 512u);
+                            va[0] = loA.x;
+                            va[1] = loA.y;
+                            vb[0] = loB.x;
+                            vb[1] = loB.y;
+                        }
+                        wA.x = __funnelshift_r(va[0], va[1], sh);
+                        wA.y = __funnelshift_r(va[1], va[2], sh);
+                        wB.x = __funnelshift_r(vb[0], vb[1], sh);
+                        wB.y = __funnelshift_r(vb[1], vb[2], sh);
                     }
                     const uint32_t m4 = 0x0f0f0f0fu;
                     const uint32_t a_lo0 = wA.x & m4, a_hi0 = (wA.x >> 4) & m4, a_lo1 = wA.y & m4, a_hi1 = (wA.y >> 4) & m4;
@@ -439,6 +457,25 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
                         }
                     }
                 }
+            };
+            if (!MIS) {
+#pragma unroll
+                for (int s = 0; s < 4; ++s) chunk(Form<0>{}, s);
+            } else if (c + 4u <= c_stop) {
+                if (wm == 0) {
+#pragma unroll
+                    for (int s = 0; s < 4; ++s) chunk(Form<0>{}, s);
+                } else if (!(wm & 4u)) {
+#pragma unroll
+                    for (int s = 0; s < 4; ++s) chunk(Form<MIS ? 1 : 0>{}, s);
+                } else {
+#pragma unroll
+                    for (int s = 0; s < 4; ++s) chunk(Form<MIS ? 2 : 0>{}, s);
+                }
+            } else {
+#pragma unroll
+                for (int s = 0; s < 3; ++s)
+                    if (c + s < c_stop) chunk(Form<MIS ? 3 : 0>{}, s);
             }
             __syncwarp();  // every lane is done with the half before it is refilled
             request_quad(half);

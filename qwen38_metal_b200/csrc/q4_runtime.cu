@@ -245,6 +245,23 @@ bool rows_byte_addressed(const Resolved *jobs, uint32_t n_jobs, uint32_t groups)
     return false;
 }
 
+// Single rows that run as a one-phase program of the persistent kernel instead of the short-batch kernel: plain output, K a
+// multiple of 512, byte-addressed weights, and either at least kInlineMinTiles 16-row tiles or fewer than kInlineMaxTiles.
+// Many tiles (lm_head): its 16-byte reads of the weights pay there, 248320 x 5120 at a byte offset takes 145 us against 151 in
+// a graph of calls; at 65536 rows it is 47.0 against 45.1, for a decode layer's nine projections 40.3 against 37.6.
+// Few tiles: not for speed (5120 x 5120 takes 13.3 us against 8.6). It sums in the decode chain's order, so a small stack run
+// launch by launch repeats the chain to the last bit, and the comparison of the two is only as tight as that: bf16
+// roundings between stages turn any other order into differences of 2e-3 to 4e-3 after three layers.
+// Aligned weights are faster in the short-batch kernel at every size (248320 rows 119 us against 124).
+constexpr uint32_t kInlineMinTiles = 8192, kInlineMaxTiles = 1024;
+bool single_row_inline(const q4b_runtime *rt, uint64_t m, uint64_t k, const std::vector<Resolved> &jobs, uint32_t flags) {
+    if (m != 1 || (flags & Q4B_FLAG_ACCUMULATE) || !rt->inline_max_halfs || k % 512 != 0 || k > rt->inline_max_halfs || k > q4k_stack_max_k()) return false;
+    if (rt->rows_max_m == 0) return true;  // the short-batch kernel is switched off
+    uint64_t tiles = 0;
+    for (const Resolved &r : jobs) tiles += (r.n + 15u) / 16u;
+    return (tiles >= kInlineMinTiles || tiles < kInlineMaxTiles) && rows_byte_addressed(jobs.data(), (uint32_t)jobs.size(), (uint32_t)(k / 64));
+}
+
 int profile_open(q4b_runtime *rt, cudaStream_t stream) {
     if (!rt->profiling) return Q4B_OK;
     if (rt->prof_used + 2 > rt->prof_events.size()) {
@@ -551,11 +568,10 @@ int enqueue_matmul(q4b_runtime *rt, const void *x_dev, int x_dtype, uint64_t m, 
                    const std::vector<Resolved> &jobs, float *const *outs, uint32_t flags, cudaStream_t stream) {
     const bool want_tensor = (flags & Q4B_FLAG_TENSOR) != 0, want_stream = (flags & Q4B_FLAG_STREAM) != 0;
     const size_t esize = x_dtype == Q4B_F32 ? 4 : 2;
-    // one row, K a multiple of 512, plain output: the persistent kernel (any byte offset)
-    const bool single = m == 1 && !(flags & Q4B_FLAG_ACCUMULATE) && rt->inline_max_halfs && k % 512 == 0 && k <= rt->inline_max_halfs && k <= q4k_stack_max_k();
+    const bool single = single_row_inline(rt, m, k, jobs, flags);
     // Short batches (up to rows_max_m rows; any m when the caller asks for the streaming form) run on the integer
-    // tensor-core kernel, as do single rows that the persistent kernel does not take.
-    bool rows = !want_tensor && (m >= 2 || (!single && m < rt->gemm_min_m)) && rt->rows_max_m >= 2 && (want_stream || m <= rt->rows_max_m) &&
+    // tensor-core kernel, as do single rows but for the few that the persistent kernel takes.
+    bool rows = !want_tensor && (m >= 2 || (!single && m < rt->gemm_min_m)) && rt->rows_max_m >= 1 && (want_stream || m <= rt->rows_max_m) &&
                 ((uintptr_t)x_dev & 15u) == 0;
     for (size_t j0 = 0; j0 < jobs.size() && rows; j0 += q4::kMaxJobs) {
         uint32_t tiles = 0, part_chunks = 0;
@@ -1927,7 +1943,7 @@ extern "C" int q4b_describe_dispatch(q4b_runtime *rt, int x_dtype, uint64_t m, u
     if (int st = resolve_jobs(rt, jobs, n_jobs, m, k, &resolved)) return st;
     uint32_t fast = 0;
     for (const Resolved &r : resolved) fast += job_is_fast(r, (uint32_t)(k / 64)) ? 1u : 0u;
-    if (m == 1 && rt->inline_max_halfs && k % 512 == 0 && k <= rt->inline_max_halfs && k <= q4k_stack_max_k()) {
+    if (single_row_inline(rt, m, k, resolved, 0)) {
         snprintf(text, text_len, "single_row_i8 one-phase persistent launch, jobs=%u (byte-addressed %u)", n_jobs, n_jobs - fast);
         return Q4B_OK;
     }

@@ -2,19 +2,22 @@
 // reference's batched kernels (qwen38_q4_affine_matvec_batch2/4/8, shaders/qwen38.metal:213-246 applied per row),
 // HBM-bound on B200 because every packed weight is read once for all rows.
 //
-// Arithmetic. Every affine group (64 inputs) of an activation row is held as 23-bit fixed point after an exact
-// power-of-two scaling by the group's own largest magnitude, x' = d0 + 256 d1 + 65536 d2 with signed 8-bit digits. A
-// packed weight word becomes two byte registers (even and odd nibbles) and is the A operand of mma.sync.m16n8k32.s32.u8.s8 as it is; the B operand holds one digit of eight
-// activation rows, so one MMA returns, for 16 weight rows and 8 activation rows, the exact integer sum of
-// q * digit over 32 inputs. An affine group (64 inputs) is two MMAs per digit; its three integer sums are
-// put together (q0 + 256 q1 + 65536 q2, the group's exact integer dot product, rounded to fp32 once), the power of two is
-// undone and the sum is scaled with the group's bf16 scale in fp32; the bias term is bias * (sum of x' over the group).
-// Products and group sums are exact; the approximations are the fixed-point step of the activation (2^-22 of the largest
-// of 64 neighbours, the last bit of an fp32 number of that size) and fp32 rounding of the per-group terms, as in the
-// reference. A group that holds an infinity or a NaN makes every result of its row NaN.
+// Arithmetic. Every affine group (64 inputs) of an activation row is held as fixed point after an exact power-of-two
+// scaling by the group's own largest magnitude, x' = d0 + 256 d1 + 65536 d2 (+ 2^24 d3) with D signed 8-bit digits. A packed
+// weight word becomes two byte registers (even and odd nibbles): a nibble in the upper half of a byte with its top bit
+// flipped is the signed byte 16 (q - 8), so the A operand of mma.sync.m16n8k32.s32.s8.s8 takes two logic instructions
+// and a shift for eight weights, and the weights are centred: y = scale * sum x (q - 8) + (bias + 8 scale) * sum x, whose two
+// terms do not cancel one another as those of the uncentred form do. The B operand holds one digit of eight activation
+// rows; an affine group is two MMAs per digit, and its integer sums are exact, put together with one rounding to fp32, and
+// scaled in fp32. The approximations are the fixed-point step of the activation and the fp32 rounding of the per-group terms.
+// Relative error (2-norm) of a result against 64 bits, normal inputs, K = 5120: 1.0e-7 with four digits or bf16 inputs, 3.0e-7 with three
+// digits of fp32 inputs (uncentred: 1.1e-7 to 2.2e-7, and 1.3e-7 through fp16 terms; 3.3e-7 with three digits of fp32 inputs).
+// D = 4 leaves the step at 2^-30 of the largest of 64 neighbours (an fp32 number within 2^6 of it is exact): fp32 inputs of up
+// to four rows, and byte-addressed ones. D = 3, at 2^-22, is exact for bf16 numbers within 2^14. A group that holds an
+// infinity or a NaN makes every result of its row NaN.
 //
-// Up to four rows (DC) the three digits of two rows share one B operand -- columns 0..2 hold the digits of the first row,
-// 4..6 those of the second -- instead of one digit of eight rows each: 2 MMAs per group and pair of rows where the form
+// Up to four rows (DC) the digits of two rows share one B operand -- columns 0..3 hold the digits of the first row,
+// 4..7 those of the second (three digits leave the last of the four zero) -- instead of one digit of eight rows each: 2 MMAs per group and pair of rows where the form
 // above takes 6 for up to eight.
 //
 // Work. The K range is cut into `parts` runs of 128-input chunks. A block holds the digits of ONE part for all rows
@@ -37,8 +40,8 @@
 // kernel that lets a dependent start early ever writes -- and only then waits for the kernel before it.
 // What bounds it and what was measured (B200, a graph of calls, one call; in brackets the ring of single chunks with a rolled
 // loop, which issued 162 warp instructions a chunk where 100 will do): 4 rows x 34816 x 5120 24.3 us = 4.1 TB/s (26.0), 4 rows x
-// 248320 x 5120 129 us = 5.5 TB/s (147), 8 fp32 rows x 8192 x 5120 at a byte offset 16.3 us (18.5), one fp32 row x 5120 x 17408 at a
-// byte offset 16.6 us (20.1), 16 rows x 34816 x 5120 63 us (67). Eight rows x 34816 x 5120 take 31.1 us; a form that walked two
+// 248320 x 5120 129 us = 5.5 TB/s (147), 8 fp32 rows x 8192 x 5120 at a byte offset 17.7 us (18.5), one fp32 row x 5120 x 17408 at a
+// byte offset 17.1 us (20.1), 16 rows x 34816 x 5120 63 us (67). Eight rows x 34816 x 5120 take 31.1 us; a form that walked two
 // tiles at a time took 28.8 there and lost everywhere else. Small calls are bound by launch, conversion and the first round
 // trips (2.5 us until the digits are ready, 2 us for the contributions to meet), long ones by the warps' instruction issue.
 // Requesting the second half of the ring only after the activation is out costs 0.6 us in a row of calls and gains nothing.
@@ -64,20 +67,21 @@ __host__ __device__ constexpr uint32_t rows_half_bytes(bool mis) { return rows_w
 __host__ __device__ constexpr bool rows_dc(uint32_t m) { return m <= kRowsPairColumns; }
 __host__ __device__ constexpr uint32_t rows_padded(uint32_t m) { return rows_dc(m) ? (m + 1u) & ~1u : (m + 7u) & ~7u; }
 
-// Shared memory of one chunk's digits: [group 2][digit 3][activation row MP][64 bytes], DC: [group 2][row MP][digit 3][64 bytes]. The 64 bytes of a (group, digit,
+// Shared memory of one chunk's digits: [group 2][digit D][activation row MP][64 bytes], DC: [group 2][row MP][digit D][64 bytes]. The 64 bytes of a (group, digit,
 // row) hold the 64 inputs of the group in the order lane t of a quad wants them as B registers of the group's two MMAs:
 // byte 16 t + 8 j + 4 odd + i  <->  input 16 t + 8 j + 2 i + odd   (t: quad lane, j: MMA of the group, i: byte).
-__host__ __device__ constexpr uint32_t rows_chunk_bytes(uint32_t mp) { return 2u * 3u * mp * 64u; }
+__host__ __device__ constexpr uint32_t rows_chunk_bytes(uint32_t mp, uint32_t digits) { return 2u * digits * mp * 64u; }
+__host__ __device__ constexpr uint32_t rows_digits(uint32_t m, bool mis, bool f32) { return f32 && (rows_dc(m) || mis) ? 4u : 3u; }
 
 // beside the digits: {sum of x', 2^-e} of every group and row, rows in pairs: {sum, sum, 2^-e, 2^-e}; DC: what a lane
-// multiplies digits 0 and 1 with and what digit 2: {sum, 2^-e, 0, 2^(16-e)}
+// multiplies digits 0 and 1 with and what digits 2 and 3: {0, 2^-e, sum, 2^(16-e)} -- the sum beside the digits that weigh
 __host__ __device__ constexpr uint32_t rows_scale_bytes(bool dc) { return dc ? 16u : 8u; }
-__host__ __device__ inline size_t rows_smem_bytes(uint32_t mp, uint32_t part_chunks, bool mis, bool dc) {
-    return (size_t)kRowsWarps * 2u * rows_half_bytes(mis) + (size_t)part_chunks * (rows_chunk_bytes(mp) + 2u * mp * rows_scale_bytes(dc));
+__host__ __device__ inline size_t rows_smem_bytes(uint32_t mp, uint32_t part_chunks, bool mis, bool dc, uint32_t digits) {
+    return (size_t)kRowsWarps * 2u * rows_half_bytes(mis) + (size_t)part_chunks * (rows_chunk_bytes(mp, digits) + 2u * mp * rows_scale_bytes(dc));
 }
 
-// Sums are carried 2^12 too small: a group's sum over 64 inputs times 0..15 of the largest fp32 numbers stays finite.
-constexpr float kRowsSumScale = 1.0f / 4096.0f;
+// Sums are carried 2^16 too small (2^12 with the weights' 16): a group's sum over 64 of the largest fp32 numbers stays finite.
+constexpr float kRowsSumScale = 1.0f / 65536.0f;
 
 // 16 bytes starting `mis` (0..15, any value per lane) bytes into the 32-byte window {lo, hi}
 __device__ __forceinline__ uint4 realign_16_any(const uint4 &lo, const uint4 &hi, uint32_t mis) {
@@ -90,9 +94,9 @@ __device__ __forceinline__ uint4 realign_16_any(const uint4 &lo, const uint4 &hi
     return make_uint4(__funnelshift_r(v[0], v[1], sh), __funnelshift_r(v[1], v[2], sh), __funnelshift_r(v[2], v[3], sh), __funnelshift_r(v[3], v[4], sh));
 }
 
-// exponent that puts a group's largest magnitude into [2^21, 2^22); both 2^e and 2^-e are normal numbers. Magnitudes
-// below 2^-105 keep an absolute step of 2^-126.
-__device__ __forceinline__ int rows_group_exponent(uint32_t amax_bits) { return min(126, 148 - (int)(amax_bits >> 23)); }
+// Exponent that puts a group's largest magnitude into [2^21, 2^22), or with four digits into [2^29, 2^30); both 2^e and 2^-e
+// are normal numbers. Magnitudes below 2^-105 (2^-97) keep an absolute step of 2^-126.
+__device__ __forceinline__ int rows_group_exponent(uint32_t amax_bits, int digits) { return min(126, (digits == 4 ? 156 : 148) - (int)(amax_bits >> 23)); }
 
 __device__ __forceinline__ unsigned long long rows_ns() {
     unsigned long long t;
@@ -105,7 +109,7 @@ struct Form {
     static constexpr int value = F;
 };
 
-template <int NB, bool DC, bool MIS>
+template <int NB, bool DC, bool MIS, int D>
 __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __grid_constant__ RowsParams p) {
     constexpr uint32_t MP = (DC ? 2 : 8) * NB;
     constexpr uint32_t T = kRowsWarps * 32;
@@ -117,7 +121,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
     // parts begin at multiples of four chunks: parameters are copied in 16-byte pieces of eight groups
     const uint32_t c_lo = q4_rows_part_begin(p.cpt, p.parts, part), c_hi = q4_rows_part_begin(p.cpt, p.parts, part + 1u), nch = c_hi - c_lo;
     uint8_t *xdig = smem + kRowsWarps * 2u * kHalf;
-    float *xscale = reinterpret_cast<float *>(xdig + (size_t)p.part_chunks * rows_chunk_bytes(MP));
+    float *xscale = reinterpret_cast<float *>(xdig + (size_t)p.part_chunks * rows_chunk_bytes(MP, D));
     const uint32_t ring = (uint32_t)__cvta_generic_to_shared(smem) + warp * 2u * kHalf;
 
     // ---- a tile's weights: lane l copies 16 bytes of row l >> 2 (and of the row eight further down) per chunk. The four 16-byte quarters of a row are stored with quarter q at q ^ (2 * bit 1 of the row), so
@@ -247,11 +251,11 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
         }
     };
     auto digits_at = [&](uint32_t chunk, uint32_t grp, uint32_t mrow) {
-        return xdig + (size_t)chunk * rows_chunk_bytes(MP) + (size_t)grp * 3u * MP * 64u + (size_t)mrow * (DC ? 192u : 64u);
+        return xdig + (size_t)chunk * rows_chunk_bytes(MP, D) + (size_t)grp * D * MP * 64u + (size_t)mrow * (DC ? D * 64u : 64u);
     };
     auto store_scale = [&](uint32_t chunk, uint32_t grp, uint32_t mrow, float sum, float inv) {
         if (DC) {
-            *reinterpret_cast<float4 *>(xscale + ((size_t)(chunk * 2u + grp) * MP + mrow) * 4u) = make_float4(sum, inv, 0.f, inv * 65536.f);
+            *reinterpret_cast<float4 *>(xscale + ((size_t)(chunk * 2u + grp) * MP + mrow) * 4u) = make_float4(0.f, inv, sum, inv * 65536.f);
         } else {
             float *dst = xscale + ((size_t)(chunk * 2u + grp) * (MP / 2u) + (mrow >> 1)) * 4u + (mrow & 1u);
             dst[0] = sum;
@@ -272,24 +276,31 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
         for (int j = 0; j < 8; ++j) mx = max(mx, __float_as_uint(v[j]) & 0x7fffffffu);
 #pragma unroll
         for (int off = 4; off > 0; off >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-        const int e = rows_group_exponent(mx);
+        const int e = rows_group_exponent(mx, D);
         const float scale = __uint_as_float((uint32_t)(e + 127) << 23), inv = __uint_as_float((uint32_t)(127 - e) << 23) * kRowsSumScale;
-        int sum = 0;
+        int sum = 0, low = 0;  // (low: the lowest byte apart where 64 inputs of 30 bits would not fit)
         uint32_t z[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             const int xi = __float2int_rn(v[j] * scale);
-            sum += xi;
-            z[j] = ((uint32_t)xi + 0x00808080u) ^ 0x00808080u;  // bytes 0..2: the signed digits
+            sum += D == 4 ? xi >> 8 : xi;
+            if (D == 4) low += xi & 0xff;
+            z[j] = ((uint32_t)xi + 0x00808080u) ^ 0x00808080u;  // bytes 0..2 (and 3): the signed digits
         }
         sum += __shfl_xor_sync(0xffffffffu, sum, 1);
         sum += __shfl_xor_sync(0xffffffffu, sum, 2);
         sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+        if (D == 4) {
+            low += __shfl_xor_sync(0xffffffffu, low, 1);
+            low += __shfl_xor_sync(0xffffffffu, low, 2);
+            low += __shfl_xor_sync(0xffffffffu, low, 4);
+        }
+        const float total = D == 4 ? fmaf((float)sum, 256.f, (float)low) : (float)sum;
         if (live) {
             const uint32_t chunk = b8 >> 4, grp = (b8 >> 3) & 1u, b = b8 & 7u;  // block b of the group: inputs 8 b .. 8 b + 7
             uint8_t *dst = digits_at(chunk, grp, mrow) + 16u * (b >> 1) + 8u * (b & 1u);
 #pragma unroll
-            for (int d = 0; d < 3; ++d) {
+            for (int d = 0; d < D; ++d) {
                 const uint32_t sel = (uint32_t)d | ((4u + (uint32_t)d) << 4);
                 uint2 w;
                 w.x = __byte_perm(__byte_perm(z[0], z[2], sel), __byte_perm(z[4], z[6], sel), 0x5410u);  // even inputs
@@ -297,7 +308,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
                 *reinterpret_cast<uint2 *>(dst + (size_t)d * (DC ? 64u : MP * 64u)) = w;
             }
             // infinity or NaN: poison the row
-            if (b == 0) store_scale(chunk, grp, mrow, mx >= 0x7f800000u ? __uint_as_float(0x7fc00000u) : (float)sum * inv, inv);
+            if (b == 0) store_scale(chunk, grp, mrow, mx >= 0x7f800000u ? __uint_as_float(0x7fc00000u) : total * inv, inv);
         }
     }
     __syncthreads();
@@ -306,11 +317,11 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
 
     // ---- tiles ----
     // B operands: digit d of row g of a block of eight (16 bytes from lane t); DC: digit g & 3 of row g >> 2 of a pair, zeros
-    // in columns 3 and 7 and in those of a row past m
-    auto has_x = [&](int nb) { return (g & 3u) < 3u && nb * 2u + (g >> 2) < p.m; };
-    const uint32_t xdig_addr = (uint32_t)__cvta_generic_to_shared(xdig) + (DC ? (g >> 2) * 192u + (g & 3u) * 64u : g * 64u) + t * 16u;
+    // in the columns of a fourth digit that there is not and of a row past m
+    auto has_x = [&](int nb) { return (g & 3u) < (uint32_t)D && nb * 2u + (g >> 2) < p.m; };
+    const uint32_t xdig_addr = (uint32_t)__cvta_generic_to_shared(xdig) + (DC ? (g >> 2) * (D * 64u) + (g & 3u) * 64u : g * 64u) + t * 16u;
     const uint32_t xscale_addr = (uint32_t)__cvta_generic_to_shared(xscale) + (DC ? (t >> 1) * 16u + (t & 1u) * 8u : t * 16u);
-    constexpr int XD = DC ? 1 : 3;  // B operands of a group and block of rows
+    constexpr int XD = DC ? 1 : D;  // B operands of a group and block of rows
     uint4 xf[2][NB][XD];
 #pragma unroll
     for (int i = 0; i < 2 * NB * XD; ++i) (&xf[0][0][0])[i] = make_uint4(0, 0, 0, 0);
@@ -343,7 +354,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
         float acc[NB][AV];
 #pragma unroll
         for (int i = 0; i < NB * AV; ++i) (&acc[0][0])[i] = 0.f;
-        uint32_t xc = xdig_addr + (c_begin - c_lo) * rows_chunk_bytes(MP);
+        uint32_t xc = xdig_addr + (c_begin - c_lo) * rows_chunk_bytes(MP, D);
         uint32_t xs = xscale_addr + (c_begin - c_lo) * (2u * MP * rows_scale_bytes(DC));
         for (uint32_t c = c_begin; c < c_stop; c += 4u) {
             cp_async_wait<1>();
@@ -379,14 +390,14 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
                     uint4 xv[NB];  // {sum, sum, 2^-e, 2^-e} of rows 2 t, 2 t + 1 of this block of 8; DC: {sum, factor} of this lane
 #pragma unroll
                     for (int nb = 0; nb < NB; ++nb) {
-                        const uint32_t xcs = xc + s * rows_chunk_bytes(MP), xss = xs + s * (2u * MP * rows_scale_bytes(DC));
+                        const uint32_t xcs = xc + s * rows_chunk_bytes(MP, D), xss = xs + s * (2u * MP * rows_scale_bytes(DC));
                         if constexpr (DC) {
-                            lds_v4_keep(xf[grp][nb][0], xcs + (uint32_t)(grp * 3 * MP * 64 + nb * 384), has_x(nb));
+                            lds_v4_keep(xf[grp][nb][0], xcs + (uint32_t)(grp * D * MP * 64 + nb * 2 * D * 64), has_x(nb));
                             const uint2 f = lds_v2(xss + (uint32_t)((grp * MP + nb * 2) * 16));
                             xv[nb] = make_uint4(f.x, f.y, 0, 0);
                         } else {
 #pragma unroll
-                            for (int d = 0; d < XD; ++d) xf[grp][nb][d] = lds_v4(xcs + (uint32_t)((grp * 3 + d) * MP + nb * 8) * 64u);
+                            for (int d = 0; d < XD; ++d) xf[grp][nb][d] = lds_v4(xcs + (uint32_t)((grp * D + d) * MP + nb * 8) * 64u);
                             xv[nb] = lds_v4(xss + (uint32_t)(grp * MP + nb * 8) * 8u);
                         }
                     }
@@ -420,11 +431,13 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
                         wB.x = __funnelshift_r(vb[0], vb[1], sh);
                         wB.y = __funnelshift_r(vb[1], vb[2], sh);
                     }
-                    const uint32_t m4 = 0x0f0f0f0fu;
-                    const uint32_t a_lo0 = wA.x & m4, a_hi0 = (wA.x >> 4) & m4, a_lo1 = wA.y & m4, a_hi1 = (wA.y >> 4) & m4;
-                    const uint32_t b_lo0 = wB.x & m4, b_hi0 = (wB.x >> 4) & m4, b_lo1 = wB.y & m4, b_hi1 = (wB.y >> 4) & m4;
+                    const uint32_t up = 0xf0f0f0f0u, flip = 0x80808080u;
+                    const uint32_t a_lo0 = ((wA.x << 4) & up) ^ flip, a_hi0 = (wA.x & up) ^ flip, a_lo1 = ((wA.y << 4) & up) ^ flip, a_hi1 = (wA.y & up) ^ flip;
+                    const uint32_t b_lo0 = ((wB.x << 4) & up) ^ flip, b_hi0 = (wB.x & up) ^ flip, b_lo1 = ((wB.y << 4) & up) ^ flip, b_hi1 = (wB.y & up) ^ flip;
                     const float sa = __uint_as_float(grp ? pr[0] & 0xffff0000u : pr[0] << 16), sb = __uint_as_float(grp ? pr[1] & 0xffff0000u : pr[1] << 16);
-                    const float ba = __uint_as_float(grp ? pr[2] & 0xffff0000u : pr[2] << 16), bb = __uint_as_float(grp ? pr[3] & 0xffff0000u : pr[3] << 16);
+                    // (the MMAs' weights are 16 (q - 8): everything is carried 16 times too large until the end of the tile)
+                    const float ba = fmaf(8.f, sa, __uint_as_float(grp ? pr[2] & 0xffff0000u : pr[2] << 16)) * 16.f;
+                    const float bb = fmaf(8.f, sb, __uint_as_float(grp ? pr[3] & 0xffff0000u : pr[3] << 16)) * 16.f;
 #pragma unroll
                     for (int nb = 0; nb < NB; ++nb) {
                         int q[XD][4];
@@ -432,20 +445,21 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
                         for (int d = 0; d < XD; ++d) {
                             const uint4 &x = xf[grp][nb][d];
                             q[d][0] = q[d][1] = q[d][2] = q[d][3] = 0;
-                            mma_u8s8_16832(q[d], a_lo0, b_lo0, a_hi0, b_hi0, x.x, x.y);
-                            mma_u8s8_16832(q[d], a_lo1, b_lo1, a_hi1, b_hi1, x.z, x.w);
+                            mma_s8s8_16832(q[d], a_lo0, b_lo0, a_hi0, b_hi0, x.x, x.y);
+                            mma_s8s8_16832(q[d], a_lo1, b_lo1, a_hi1, b_hi1, x.z, x.w);
                         }
                         if constexpr (DC) {
-                            // even lanes hold digits 0 and 1 of a row, odd ones digit 2 (and a zero); the two sums meet at
-                            // the end of the tile
+                            // even lanes hold digits 0 and 1 of a row, odd ones digits 2 and 3; the two sums meet at the
+                            // end of the tile
                             const float sum = __uint_as_float(xv[nb].x), f = __uint_as_float(xv[nb].y);
                             acc[nb][0] = fmaf(__int2float_rn(q[0][0] + (q[0][1] << 8)) * f, sa, fmaf(sum, ba, acc[nb][0]));
                             acc[nb][1] = fmaf(__int2float_rn(q[0][2] + (q[0][3] << 8)) * f, sb, fmaf(sum, bb, acc[nb][1]));
                         } else {
-                            // the group's integer dot product q0 + 256 q1 + 65536 q2 (exact; |q0 + 256 q1| < 2^25 is rounded to fp32 once)
+                            // the group's integer dot product: two exact sums of two digits (|q0 + 256 q1| < 2^29), put together
 #pragma unroll
                             for (int i = 0; i < 4; ++i) {
-                                const float dot = fmaf(__int2float_rn(q[XD - 1][i]), 65536.f, __int2float_rn(q[0][i] + (q[XD / 2][i] << 8))) *
+                                const int hi = D == 4 ? q[XD / 2][i] + (q[XD - 1][i] << 8) : q[XD - 1][i];
+                                const float dot = fmaf(__int2float_rn(hi), 65536.f, __int2float_rn(q[0][i] + (q[DC ? 0 : 1][i] << 8))) *
                                                   __uint_as_float((i & 1) ? xv[nb].w : xv[nb].z);
                                 acc[nb][i] = fmaf(dot, i < 2 ? sa : sb, acc[nb][i]);
                             }
@@ -480,7 +494,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
             __syncwarp();  // every lane is done with the half before it is refilled
             request_quad(half);
             half ^= 1u;
-            xc += 4u * rows_chunk_bytes(MP);
+            xc += 4u * rows_chunk_bytes(MP, D);
             xs += 4u * (2u * MP * rows_scale_bytes(DC));
         }
         if (tr && first_run) tr[2] = rows_ns();
@@ -492,7 +506,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
             for (int i = 0; i < NB * AV; ++i) (&acc[0][0])[i] += __shfl_xor_sync(0xffffffffu, (&acc[0][0])[i], 1);
         }
 #pragma unroll
-        for (int i = 0; i < NB * AV; ++i) (&acc[0][0])[i] *= 1.0f / kRowsSumScale;
+        for (int i = 0; i < NB * AV; ++i) (&acc[0][0])[i] *= 1.0f / (16.0f * kRowsSumScale);
         // value i of a block of rows: activation row and weight row of the tile (DC: only even lanes store)
         auto act_row = [&](int nb, int i) { return DC ? nb * 2u + (t >> 1) : nb * 8u + 2u * t + (uint32_t)(i & 1); };
         auto weight_row = [&](int i) { return g + 8u * (uint32_t)(DC ? i : i >> 1); };
@@ -572,32 +586,35 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
 
 // Largest part (in chunks) a block can hold for `mp` padded activation rows, 0 if not even
 // four chunks fit.
-static uint32_t rows_part_capacity(uint32_t mp, bool mis, bool dc) {
+static uint32_t rows_part_capacity(uint32_t mp, bool mis, bool dc, uint32_t digits) {
     int dev = 0, optin = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
     uint32_t chunks = 0;
-    while (q4::rows_smem_bytes(mp, chunks + 1, mis, dc) <= (size_t)optin && (chunks + 1) * mp <= 256u) ++chunks;
+    while (q4::rows_smem_bytes(mp, chunks + 1, mis, dc, digits) <= (size_t)optin && (chunks + 1) * mp <= 256u) ++chunks;
     return chunks >= 4 ? chunks : 0;
 }
+
+// Activation rows a launch takes: 16, or 8 where they are held with four digits.
+extern "C" uint32_t q4k_rows_per_launch(int mis, int f32) { return mis && f32 ? 8u : 16u; }
 
 // How the K range of a launch is cut: the number of parts (0: the shape is not supported) and the longest part. `mis`: the
 // byte-addressed instance, which any K % 64 == 0 and any byte offset may use; the other one wants K % 512 == 0 and
 // 16-byte alignment.
-extern "C" uint32_t q4k_rows_plan(uint32_t m, uint32_t k, uint32_t tiles, uint32_t sm_count, int mis, uint32_t *part_chunks) {
-    if (m < 1 || m > 16 || k == 0 || k % (mis ? 64u : 512u) != 0 || tiles == 0) return 0;
+extern "C" uint32_t q4k_rows_plan(uint32_t m, uint32_t k, uint32_t tiles, uint32_t sm_count, int mis, int f32, uint32_t *part_chunks) {
+    if (m < 1 || m > q4k_rows_per_launch(mis, f32) || k == 0 || k % (mis ? 64u : 512u) != 0 || tiles == 0) return 0;
     const uint32_t mp = q4::rows_padded(m);
-    const uint32_t cap = rows_part_capacity(mp, mis != 0, q4::rows_dc(m));
+    const uint32_t cap = rows_part_capacity(mp, mis != 0, q4::rows_dc(m), q4::rows_digits(m, mis != 0, f32 != 0));
     return cap ? q4_rows_plan((k / 64u + 1u) / 2u, tiles, sm_count, cap, 1u, mp, part_chunks, nullptr) : 0u;
 }
 
 extern "C" uint32_t q4k_rows_padded(uint32_t m) { return q4::rows_padded(m); }
 
-template <int NB, bool DC, bool MIS>
+template <int NB, bool DC, bool MIS, int D>
 static cudaError_t rows_launch(const q4::RowsParams &p, uint32_t grid, size_t smem, cudaStream_t stream) {
-    const cudaError_t e = cudaFuncSetAttribute(q4::q4_rows_kernel<NB, DC, MIS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = cudaFuncSetAttribute(q4::q4_rows_kernel<NB, DC, MIS, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
@@ -609,18 +626,22 @@ static cudaError_t rows_launch(const q4::RowsParams &p, uint32_t grid, size_t sm
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, q4::q4_rows_kernel<NB, DC, MIS>, p);
+    return cudaLaunchKernelEx(&cfg, q4::q4_rows_kernel<NB, DC, MIS, D>, p);
 }
 
 extern "C" cudaError_t q4k_rows(const q4::RowsParams *params, uint32_t sm_count, cudaStream_t stream) {
     const q4::RowsParams &p = *params;
     const uint32_t mp = q4::rows_padded(p.m);
     const bool mis = p.byte_addressed != 0, dc = q4::rows_dc(p.m);
-    const size_t smem = q4::rows_smem_bytes(mp, p.part_chunks, mis, dc);
+    const uint32_t digits = q4::rows_digits(p.m, mis, p.x_is_f32 != 0);
+    const size_t smem = q4::rows_smem_bytes(mp, p.part_chunks, mis, dc, digits);
     const uint32_t grid = (sm_count / p.parts) * p.parts;
-    if (grid == 0 || p.run == 0) return cudaErrorInvalidValue;
-    if (mp == 2) return mis ? rows_launch<1, true, true>(p, grid, smem, stream) : rows_launch<1, true, false>(p, grid, smem, stream);
-    if (mp == 4) return mis ? rows_launch<2, true, true>(p, grid, smem, stream) : rows_launch<2, true, false>(p, grid, smem, stream);
-    if (mp == 16) return mis ? rows_launch<2, false, true>(p, grid, smem, stream) : rows_launch<2, false, false>(p, grid, smem, stream);
-    return mis ? rows_launch<1, false, true>(p, grid, smem, stream) : rows_launch<1, false, false>(p, grid, smem, stream);
+    if (grid == 0 || p.run == 0 || p.m > q4k_rows_per_launch(mis, (int)p.x_is_f32)) return cudaErrorInvalidValue;
+    if (mp == 2 && digits == 4) return mis ? rows_launch<1, true, true, 4>(p, grid, smem, stream) : rows_launch<1, true, false, 4>(p, grid, smem, stream);
+    if (mp == 2) return mis ? rows_launch<1, true, true, 3>(p, grid, smem, stream) : rows_launch<1, true, false, 3>(p, grid, smem, stream);
+    if (mp == 4 && digits == 4) return mis ? rows_launch<2, true, true, 4>(p, grid, smem, stream) : rows_launch<2, true, false, 4>(p, grid, smem, stream);
+    if (mp == 4) return mis ? rows_launch<2, true, true, 3>(p, grid, smem, stream) : rows_launch<2, true, false, 3>(p, grid, smem, stream);
+    if (mp == 16) return mis ? rows_launch<2, false, true, 3>(p, grid, smem, stream) : rows_launch<2, false, false, 3>(p, grid, smem, stream);
+    if (digits == 4) return rows_launch<1, false, true, 4>(p, grid, smem, stream);
+    return mis ? rows_launch<1, false, true, 3>(p, grid, smem, stream) : rows_launch<1, false, false, 3>(p, grid, smem, stream);
 }

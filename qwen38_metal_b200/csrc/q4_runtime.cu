@@ -500,12 +500,12 @@ int enqueue_gemm(q4b_runtime *rt, const void *x_dev, int x_dtype, uint64_t m, ui
 // conditions (the caller falls back to the general streaming kernel), else a status.
 int launch_rows(q4b_runtime *rt, const void *x_dev, int x_dtype, uint32_t m, uint32_t k, const Resolved *jobs, uint32_t n_jobs,
                 float *const *outs, uint32_t flags, cudaStream_t stream) {
-    if (m < 1 || m > 16 || ((uintptr_t)x_dev & 15u)) return -1;
+    if (m < 1 || ((uintptr_t)x_dev & 15u)) return -1;
     uint32_t tiles = 0;
     for (uint32_t i = 0; i < n_jobs; ++i) tiles += (jobs[i].n + 15u) / 16u;
     const int mis = rows_byte_addressed(jobs, n_jobs, k / 64u) ? 1 : 0;
     uint32_t part_chunks = 0;
-    const uint32_t parts = q4k_rows_plan(m, k, tiles, (uint32_t)rt->sm_count, mis, &part_chunks);
+    const uint32_t parts = q4k_rows_plan(m, k, tiles, (uint32_t)rt->sm_count, mis, x_dtype == Q4B_F32, &part_chunks);
     if (parts == 0) return -1;
     q4::RowsParams p;
     memset(&p, 0, sizeof p);
@@ -573,22 +573,24 @@ int enqueue_matmul(q4b_runtime *rt, const void *x_dev, int x_dtype, uint64_t m, 
     // tensor-core kernel, as do single rows but for the few that the persistent kernel takes.
     bool rows = !want_tensor && (m >= 2 || (!single && m < rt->gemm_min_m)) && rt->rows_max_m >= 1 && (want_stream || m <= rt->rows_max_m) &&
                 ((uintptr_t)x_dev & 15u) == 0;
+    uint32_t rows_step = rt->rows_max_m;  // rows per launch
     for (size_t j0 = 0; j0 < jobs.size() && rows; j0 += q4::kMaxJobs) {
         uint32_t tiles = 0, part_chunks = 0;
         const uint32_t nj = (uint32_t)std::min(jobs.size() - j0, (size_t)q4::kMaxJobs);
         for (size_t j = j0; j < j0 + nj; ++j) tiles += (jobs[j].n + 15u) / 16u;
         const int mis = rows_byte_addressed(&jobs[j0], nj, (uint32_t)(k / 64)) ? 1 : 0;
-        const uint32_t full = (uint32_t)(m < rt->rows_max_m ? m : rt->rows_max_m), rest = (uint32_t)(m % rt->rows_max_m);
+        rows_step = std::min(rows_step, q4k_rows_per_launch(mis, x_dtype == Q4B_F32));
         if (mis && !want_stream && m >= rt->gemm_min_m) {
             rows = false;
             break;
         }
-        rows = q4k_rows_plan(full, (uint32_t)k, tiles, (uint32_t)rt->sm_count, mis, &part_chunks) != 0 &&
-               (m <= rt->rows_max_m || rest == 0 || q4k_rows_plan(rest, (uint32_t)k, tiles, (uint32_t)rt->sm_count, mis, &part_chunks) != 0);
+        const uint32_t full = (uint32_t)std::min<uint64_t>(m, rows_step), rest = (uint32_t)(m % rows_step);
+        rows = q4k_rows_plan(full, (uint32_t)k, tiles, (uint32_t)rt->sm_count, mis, x_dtype == Q4B_F32, &part_chunks) != 0 &&
+               (m <= rows_step || rest == 0 || q4k_rows_plan(rest, (uint32_t)k, tiles, (uint32_t)rt->sm_count, mis, x_dtype == Q4B_F32, &part_chunks) != 0);
     }
     if (rows) {
-        for (uint64_t m0 = 0; m0 < m; m0 += rt->rows_max_m) {
-            const uint32_t mb = (uint32_t)((m - m0) < rt->rows_max_m ? (m - m0) : rt->rows_max_m);
+        for (uint64_t m0 = 0; m0 < m; m0 += rows_step) {
+            const uint32_t mb = (uint32_t)std::min<uint64_t>(m - m0, rows_step);
             const uint8_t *xb = (const uint8_t *)x_dev + m0 * k * esize;
             for (size_t j0 = 0; j0 < jobs.size(); j0 += q4::kMaxJobs) {
                 const uint32_t nj = (uint32_t)((jobs.size() - j0) < (size_t)q4::kMaxJobs ? (jobs.size() - j0) : (size_t)q4::kMaxJobs);
@@ -1950,8 +1952,9 @@ extern "C" int q4b_describe_dispatch(q4b_runtime *rt, int x_dtype, uint64_t m, u
     if (m <= rt->rows_max_m && (fast == n_jobs || m < rt->gemm_min_m)) {
         uint32_t tiles = 0, part_chunks = 0;
         for (const Resolved &r : resolved) tiles += (r.n + 15u) / 16u;
-        const uint32_t mb = (uint32_t)(m < rt->rows_max_m ? m : rt->rows_max_m);
-        const uint32_t parts = q4k_rows_plan(mb, (uint32_t)k, tiles, (uint32_t)rt->sm_count, fast == n_jobs ? 0 : 1, &part_chunks);
+        const int mis = fast == n_jobs ? 0 : 1, f32 = x_dtype == Q4B_F32;
+        const uint32_t mb = (uint32_t)std::min<uint64_t>(m, std::min(rt->rows_max_m, q4k_rows_per_launch(mis, f32)));
+        const uint32_t parts = q4k_rows_plan(mb, (uint32_t)k, tiles, (uint32_t)rt->sm_count, mis, f32, &part_chunks);
         if (parts) {
             snprintf(text, text_len, "rows_i8 (short batch, integer tensor cores) rows_per_launch=%u k_parts=%u chunks_per_part=%u jobs=%u (a 16-byte aligned activation is assumed)",
                      mb, parts, part_chunks, n_jobs);

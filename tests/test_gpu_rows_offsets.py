@@ -69,3 +69,15 @@ def test_outliers_and_non_finite_inputs(runtime, oracle, offset):
     for r in range(3):
         assert oracle.rel_l2(out[r], ref[r]) <= 1e-5, r
     assert not np.isfinite(out[3:]).any()
+
+
+@pytest.mark.parametrize("m,offset", [(1, 0), (2, 0), (4, 2), (8, 2), (12, 6)])
+def test_fp32_inputs_keep_their_bits(runtime, oracle, m, offset):
+    """fp32 inputs in four digits: what is left is the fp32 accumulation of K / 64 groups, two roundings of 2^-24 each, which
+    add up to about sqrt(2 K / 64) 2^-24 / sqrt(3) = 1.9e-7 (three digits alone would leave 3e-7)."""
+    n, k = 256, 1024
+    trip = oracle.synth_q4(SEED, 80, n, k)
+    job = upload_matrix(runtime, *trip, offset=offset)
+    x = np.random.default_rng(m).standard_normal((m, k)).astype(np.float32)
+    out = runtime.q4_affine_matmul_mapped_batch(x.reshape(-1), m, [job])[0]
+    assert oracle.rel_l2(out.reshape(m, n), oracle.matmul_f64(x, *trip, n)) <= 1.9e-7

@@ -725,8 +725,8 @@ extern "C" int q4b_runtime_create(int device_ordinal, q4b_runtime **out) {
     if (e == cudaSuccess) e = cudaMemset(rt->counters.ptr, 0, rt->counters.capacity);
     if (e == cudaSuccess) e = rt->error_flag.ensure(256);
     if (e == cudaSuccess) e = cudaMemset(rt->error_flag.ptr, 0, rt->error_flag.capacity);
-    // enough for a decode layer's projections of a few rows; larger launches grow it
-    if (e == cudaSuccess) e = rt->rows_partials.ensure((size_t)4 << 20);
+    // enough for lm_head of four rows, 248320 wide; larger launches grow it
+    if (e == cudaSuccess) e = rt->rows_partials.ensure((size_t)8 << 20);
     if (e == cudaSuccess) e = rt->rows_counters.ensure(16384 * 4);
     if (e == cudaSuccess) e = cudaMemset(rt->rows_counters.ptr, 0, rt->rows_counters.capacity);
     if (const char *unf = getenv("Q4B_MLP_UNFUSED")) rt->mlp_unfused = strtol(unf, nullptr, 10) != 0;

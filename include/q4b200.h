@@ -17,7 +17,9 @@
  *   - `_device` twins take device pointers and a cudaStream_t (passed as void*), enqueue
  *     work and return without synchronising. They use the runtime's scratch buffers: calls
  *     on one runtime must be ordered on the device (one stream, or events). Scratch grows on
- *     first use of a larger shape, so run a shape once before capturing it in a CUDA graph;
+ *     first use of a larger shape, so run a shape once before capturing it in a CUDA graph.
+ *     Scratch that a later, larger call outgrows stays allocated until q4b_runtime_destroy, so
+ *     a captured graph may be replayed until then, ordered with the runtime's other calls;
  *   - weights are uploaded byte for byte (no expansion, no repacking, file offsets kept), so
  *     a tensor that is misaligned in its safetensors shard is misaligned in HBM; the kernels
  *     take any byte alignment.

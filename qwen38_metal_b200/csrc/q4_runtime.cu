@@ -57,10 +57,14 @@ int fail_cuda(cudaError_t e, const char *what) {
     } while (0)
 
 // Grow-only scratch buffer, power-of-two capacity: ensure_private_buffer /
-// shared_reusable_buffer of the reference (src/metal_runtime.rs:8993-9057).
+// shared_reusable_buffer of the reference (src/metal_runtime.rs:8993-9057). A block that has become too small is kept
+// until release(): a CUDA graph that was captured while it was the current one goes on using it. Capacities double, so
+// all kept blocks together are smaller than the current one.
 struct Pool {
     void *ptr = nullptr;
     size_t capacity = 0;
+    void *outgrown[64];  // (at most one per power of two)
+    int n_outgrown = 0;
     cudaError_t ensure(size_t bytes) {
         if (bytes <= capacity) return cudaSuccess;
         size_t want = 256;
@@ -68,13 +72,14 @@ struct Pool {
         void *fresh = nullptr;
         cudaError_t e = cudaMalloc(&fresh, want);
         if (e != cudaSuccess) return e;
-        if (ptr) cudaFree(ptr);
+        if (ptr) outgrown[n_outgrown++] = ptr;
         ptr = fresh;
         capacity = want;
         return cudaSuccess;
     }
     void release() {
         if (ptr) cudaFree(ptr);
+        while (n_outgrown) cudaFree(outgrown[--n_outgrown]);
         ptr = nullptr;
         capacity = 0;
     }

@@ -1,5 +1,5 @@
-// Short batches (2..16 activation rows) of MLX affine-Q4 projections on the integer tensor-core path: the shape of the
-// reference's batched kernels (qwen38_q4_affine_matvec_batch2/4/8, shaders/qwen38.metal:213-246 applied per row),
+// Single rows and short batches (up to 16 activation rows) of MLX affine-Q4 projections on the integer tensor-core path: the shape of the
+// reference's matvec and batched kernels (qwen38_q4_affine_matvec_batch2/4/8, shaders/qwen38.metal:213-246 applied per row),
 // HBM-bound on B200 because every packed weight is read once for all rows.
 //
 // Arithmetic. Every affine group (64 inputs) of an activation row is held as fixed point after an exact power-of-two
@@ -12,13 +12,17 @@
 // scaled in fp32. The approximations are the fixed-point step of the activation and the fp32 rounding of the per-group terms.
 // Relative error (2-norm) of a result against 64 bits, normal inputs, K = 5120: 1.0e-7 with four digits or bf16 inputs, 3.0e-7 with three
 // digits of fp32 inputs (uncentred: 1.1e-7 to 2.2e-7, and 1.3e-7 through fp16 terms; 3.3e-7 with three digits of fp32 inputs).
-// D = 4 leaves the step at 2^-30 of the largest of 64 neighbours (an fp32 number within 2^6 of it is exact): fp32 inputs of up
-// to four rows, and byte-addressed ones. D = 3, at 2^-22, is exact for bf16 numbers within 2^14. A group that holds an
-// infinity or a NaN makes every result of its row NaN.
+// D = 4 leaves the step at 2^-30 of the largest of 64 neighbours (bf16 within 2^22 of it is exact, fp32 within 2^6): single rows,
+// byte-addressed launches, fp32 inputs of up to four rows. D = 3, at 2^-22 (bf16 exact within 2^14), the others: 2 to 16 rows
+// of aligned tensors, where a fourth digit would cost four rows 15 % (34816 x 5120, 26.8 -> 30.8 us: a quarter more digits to
+// read). What a step costs shows when an input far above its 63 neighbours meets a weight of zero: results are off by 1e-4 (D = 3)
+// or 5e-7 (D = 4) at 10^4 times its neighbours, 1e-3 or 5e-6 at 10^5. A group that holds an infinity or a NaN makes every result of its
+// row NaN. Byte-addressed bf16 launches had three digits (and 16 rows); the fourth costs 8 rows x 34816 x 5120 47.7 -> 55.8 us, 8192 x 5120
+// 16.7 -> 17.7, 12 rows in two launches 79.6 -> 99.9 and 35.6 -> 34.2.
 //
 // Up to four rows (DC) the digits of two rows share one B operand -- columns 0..3 hold the digits of the first row,
-// 4..7 those of the second (three digits leave the last of the four zero) -- instead of one digit of eight rows each: 2 MMAs per group and pair of rows where the form
-// above takes 6 for up to eight.
+// 4..7 those of the second (three digits leave the last of the four zero) -- instead of one digit of eight rows each: 2 MMAs
+// per group and pair of rows where the form above takes 6 or 8 for up to eight.
 //
 // Work. The K range is cut into `parts` runs of 128-input chunks. A block holds the digits of ONE part for all rows
 // in shared memory (converted by the block itself from the caller's bf16 or fp32 rows). A part's work is the list of its
@@ -71,7 +75,7 @@ __host__ __device__ constexpr uint32_t rows_padded(uint32_t m) { return rows_dc(
 // row) hold the 64 inputs of the group in the order lane t of a quad wants them as B registers of the group's two MMAs:
 // byte 16 t + 8 j + 4 odd + i  <->  input 16 t + 8 j + 2 i + odd   (t: quad lane, j: MMA of the group, i: byte).
 __host__ __device__ constexpr uint32_t rows_chunk_bytes(uint32_t mp, uint32_t digits) { return 2u * digits * mp * 64u; }
-__host__ __device__ constexpr uint32_t rows_digits(uint32_t m, bool mis, bool f32) { return f32 && (rows_dc(m) || mis) ? 4u : 3u; }
+__host__ __device__ constexpr uint32_t rows_digits(uint32_t m, bool mis, bool f32) { return m == 1u || mis || (f32 && rows_dc(m)) ? 4u : 3u; }
 
 // beside the digits: {sum of x', 2^-e} of every group and row, rows in pairs: {sum, sum, 2^-e, 2^-e}; DC: what a lane
 // multiplies digits 0 and 1 with and what digits 2 and 3: {0, 2^-e, sum, 2^(16-e)} -- the sum beside the digits that weigh
@@ -598,13 +602,13 @@ static uint32_t rows_part_capacity(uint32_t mp, bool mis, bool dc, uint32_t digi
 }
 
 // Activation rows a launch takes: 16, or 8 where they are held with four digits.
-extern "C" uint32_t q4k_rows_per_launch(int mis, int f32) { return mis && f32 ? 8u : 16u; }
+extern "C" uint32_t q4k_rows_per_launch(int mis) { return mis ? 8u : 16u; }
 
 // How the K range of a launch is cut: the number of parts (0: the shape is not supported) and the longest part. `mis`: the
 // byte-addressed instance, which any K % 64 == 0 and any byte offset may use; the other one wants K % 512 == 0 and
 // 16-byte alignment.
 extern "C" uint32_t q4k_rows_plan(uint32_t m, uint32_t k, uint32_t tiles, uint32_t sm_count, int mis, int f32, uint32_t *part_chunks) {
-    if (m < 1 || m > q4k_rows_per_launch(mis, f32) || k == 0 || k % (mis ? 64u : 512u) != 0 || tiles == 0) return 0;
+    if (m < 1 || m > q4k_rows_per_launch(mis) || k == 0 || k % (mis ? 64u : 512u) != 0 || tiles == 0) return 0;
     const uint32_t mp = q4::rows_padded(m);
     const uint32_t cap = rows_part_capacity(mp, mis != 0, q4::rows_dc(m), q4::rows_digits(m, mis != 0, f32 != 0));
     return cap ? q4_rows_plan((k / 64u + 1u) / 2u, tiles, sm_count, cap, 1u, mp, part_chunks, nullptr) : 0u;
@@ -636,12 +640,13 @@ extern "C" cudaError_t q4k_rows(const q4::RowsParams *params, uint32_t sm_count,
     const uint32_t digits = q4::rows_digits(p.m, mis, p.x_is_f32 != 0);
     const size_t smem = q4::rows_smem_bytes(mp, p.part_chunks, mis, dc, digits);
     const uint32_t grid = (sm_count / p.parts) * p.parts;
-    if (grid == 0 || p.run == 0 || p.m > q4k_rows_per_launch(mis, (int)p.x_is_f32)) return cudaErrorInvalidValue;
-    if (mp == 2 && digits == 4) return mis ? rows_launch<1, true, true, 4>(p, grid, smem, stream) : rows_launch<1, true, false, 4>(p, grid, smem, stream);
-    if (mp == 2) return mis ? rows_launch<1, true, true, 3>(p, grid, smem, stream) : rows_launch<1, true, false, 3>(p, grid, smem, stream);
-    if (mp == 4 && digits == 4) return mis ? rows_launch<2, true, true, 4>(p, grid, smem, stream) : rows_launch<2, true, false, 4>(p, grid, smem, stream);
-    if (mp == 4) return mis ? rows_launch<2, true, true, 3>(p, grid, smem, stream) : rows_launch<2, true, false, 3>(p, grid, smem, stream);
-    if (mp == 16) return mis ? rows_launch<2, false, true, 3>(p, grid, smem, stream) : rows_launch<2, false, false, 3>(p, grid, smem, stream);
-    if (digits == 4) return rows_launch<1, false, true, 4>(p, grid, smem, stream);
-    return mis ? rows_launch<1, false, true, 3>(p, grid, smem, stream) : rows_launch<1, false, false, 3>(p, grid, smem, stream);
+    if (grid == 0 || p.run == 0 || p.m > q4k_rows_per_launch(mis)) return cudaErrorInvalidValue;
+    if (mis) {
+        if (mp == 2) return rows_launch<1, true, true, 4>(p, grid, smem, stream);
+        if (mp == 4) return rows_launch<2, true, true, 4>(p, grid, smem, stream);
+        return rows_launch<1, false, true, 4>(p, grid, smem, stream);
+    }
+    if (mp == 2) return digits == 4 ? rows_launch<1, true, false, 4>(p, grid, smem, stream) : rows_launch<1, true, false, 3>(p, grid, smem, stream);
+    if (mp == 4) return digits == 4 ? rows_launch<2, true, false, 4>(p, grid, smem, stream) : rows_launch<2, true, false, 3>(p, grid, smem, stream);
+    return mp == 8 ? rows_launch<1, false, false, 3>(p, grid, smem, stream) : rows_launch<2, false, false, 3>(p, grid, smem, stream);
 }

@@ -101,7 +101,7 @@ cudaError_t q4k_gemv(const q4::GemvParams *params, int column_tiles, int aligned
 uint32_t q4k_gemv_occupancy(int column_tiles, int aligned);  // resident warps per SM, 0 on error
 
 uint32_t q4k_rows_plan(uint32_t m, uint32_t k, uint32_t tiles, uint32_t sm_count, int mis, int f32, uint32_t *part_chunks);  // parts, 0: unsupported
-uint32_t q4k_rows_per_launch(int mis, int f32);
+uint32_t q4k_rows_per_launch(int mis);  // most rows of a launch
 uint32_t q4k_rows_padded(uint32_t m);  // activation rows a launch of m rows holds
 cudaError_t q4k_rows(const q4::RowsParams *params, uint32_t sm_count, cudaStream_t stream);
 

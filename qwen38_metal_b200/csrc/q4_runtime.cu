@@ -585,7 +585,7 @@ int enqueue_matmul(q4b_runtime *rt, const void *x_dev, int x_dtype, uint64_t m, 
         const uint32_t nj = (uint32_t)std::min(jobs.size() - j0, (size_t)q4::kMaxJobs);
         for (size_t j = j0; j < j0 + nj; ++j) tiles += (jobs[j].n + 15u) / 16u;
         const int mis = rows_byte_addressed(&jobs[j0], nj, (uint32_t)(k / 64)) ? 1 : 0;
-        rows_step = std::min(rows_step, q4k_rows_per_launch(mis, x_dtype == Q4B_F32));
+        rows_step = std::min(rows_step, q4k_rows_per_launch(mis));
         if (mis && !want_stream && m >= rt->gemm_min_m) {
             rows = false;
             break;
@@ -1969,7 +1969,7 @@ extern "C" int q4b_describe_dispatch(q4b_runtime *rt, int x_dtype, uint64_t m, u
         uint32_t tiles = 0, part_chunks = 0;
         for (const Resolved &r : resolved) tiles += (r.n + 15u) / 16u;
         const int mis = fast == n_jobs ? 0 : 1, f32 = x_dtype == Q4B_F32;
-        const uint32_t mb = (uint32_t)std::min<uint64_t>(m, std::min(rt->rows_max_m, q4k_rows_per_launch(mis, f32)));
+        const uint32_t mb = (uint32_t)std::min<uint64_t>(m, std::min(rt->rows_max_m, q4k_rows_per_launch(mis)));
         const uint32_t parts = q4k_rows_plan(mb, (uint32_t)k, tiles, (uint32_t)rt->sm_count, mis, f32, &part_chunks);
         if (parts) {
             snprintf(text, text_len, "rows_i8 (short batch, integer tensor cores) rows_per_launch=%u k_parts=%u chunks_per_part=%u jobs=%u (a 16-byte aligned activation is assumed)",

@@ -51,8 +51,8 @@ def test_single_row_that_adds(runtime, oracle, k, offset):
 
 @pytest.mark.parametrize("offset", [0, 2])
 def test_outliers_and_non_finite_inputs(runtime, oracle, offset):
-    """A channel a million times the rest costs the other groups no precision; an infinity or a NaN reaches every result of
-    its own row and no other row."""
+    """A channel a million times the rest costs the other groups no precision (its own group: the test below); an infinity or a
+    NaN reaches every result of its own row and no other row."""
     n, k, m = 96, 1024, 5
     trip = oracle.synth_q4(SEED, 70, n, k)
     x = np.random.default_rng(3).standard_normal((m, k)).astype(np.float32)
@@ -81,3 +81,35 @@ def test_fp32_inputs_keep_their_bits(runtime, oracle, m, offset):
     x = np.random.default_rng(m).standard_normal((m, k)).astype(np.float32)
     out = runtime.q4_affine_matmul_mapped_batch(x.reshape(-1), m, [job])[0]
     assert oracle.rel_l2(out.reshape(m, n), oracle.matmul_f64(x, *trip, n)) <= 1.9e-7
+
+
+def _zero_weight_at(trip, index):
+    """Weight zero (q = 8, bias = -8 scale) for input `index` of every group, in every row; the other weights stay live."""
+    w, s, b = trip
+    word, shift = index // 8, np.uint32(4 * (index % 8))
+    w[:, word::8] = (w[:, word::8] & ~(np.uint32(15) << shift)) | (np.uint32(8) << shift)
+    b[:] = (s + np.uint16(3 << 7)) ^ np.uint16(0x8000)  # bf16: three more in the exponent, sign flipped
+    return trip
+
+
+@pytest.mark.parametrize("spread", [1e3, 1e4, 1e5])
+@pytest.mark.parametrize("bf16", [True, False])
+@pytest.mark.parametrize("m,k,offset", [(1, 5120, 0), (1, 5120, 2), (2, 5120, 2), (3, 5184, 0), (8, 5120, 2), (13, 5120, 2), (15, 5184, 6)])
+def test_a_large_input_with_zero_weight_costs_its_neighbours_little(runtime, oracle, m, k, offset, bf16, spread):
+    """One input far above its 63 neighbours, whose own weight is zero: what is left of its group is the neighbours' sum. Bar:
+    that of the path, 1e-5. The step of four digits is 2^-30 of the power of two above the large input and inputs are off by
+    0.29 of it (rms) against a standard deviation of 1, in one group of K / 64: 2^-30 * 131072 * 0.29 / sqrt(80) = 4e-6 at
+    a spread of 1e5. Residual form, so that single rows take this kernel at every size."""
+    n = 200
+    trip = _zero_weight_at(oracle.synth_q4(SEED, 90, n, k), 37)
+    job = upload_matrix(runtime, *trip, offset=offset)
+    x = np.random.default_rng(m).standard_normal((m, k)).astype(np.float32)
+    x[:, 64 + 37] = spread
+    given = x.reshape(-1)
+    if bf16:
+        given = oracle.f32_to_bf16(given)
+        x = oracle.bf16_to_f32(given).reshape(m, k)
+    out = runtime.q4_affine_matmul_add_mapped_batch(given, m, [job], [np.zeros((m, n), dtype=np.float32)])[0].reshape(m, n)
+    ref = oracle.matmul_f64(x, *trip, n)
+    for r in range(m):
+        assert oracle.rel_l2(out[r], ref[r]) <= 1e-5, r

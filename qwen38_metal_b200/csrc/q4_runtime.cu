@@ -252,20 +252,18 @@ bool rows_byte_addressed(const Resolved *jobs, uint32_t n_jobs, uint32_t groups)
 }
 
 // Single rows that run as a one-phase program of the persistent kernel instead of the short-batch kernel: plain output, K a
-// multiple of 512, byte-addressed weights, and either at least kInlineMinTiles 16-row tiles or fewer than kInlineMaxTiles.
-// Many tiles (lm_head): its 16-byte reads of the weights pay there, 248320 x 5120 at a byte offset takes 145 us against 151 in
-// a graph of calls; at 65536 rows it is 47.0 against 45.1, for a decode layer's nine projections 40.3 against 37.6.
-// Few tiles: not for speed (5120 x 5120 takes 13.3 us against 8.6). It sums in the decode chain's order, so a small stack run
-// launch by launch repeats the chain to the last bit, and the comparison of the two is only as tight as that: bf16
-// roundings between stages turn any other order into differences of 2e-3 to 4e-3 after three layers.
-// Aligned weights are faster in the short-batch kernel at every size (248320 rows 119 us against 124).
-constexpr uint32_t kInlineMinTiles = 8192, kInlineMaxTiles = 1024;
+// multiple of 512, byte-addressed weights, at least kInlineMinTiles 16-row tiles (lm_head). Measured with weights from HBM, K = 5120,
+// this kernel against that one, in a row of calls and with a small kernel between them: 248320 rows 149 and 150 us against 151 and
+// 160, 131072 rows 84 and 85 against 84 and 92; 98304 rows 67 and 68 against 64 and 72, 65536 rows 49 and 51 against 46 and 54, a decode
+// layer's nine projections 42 and 44 against 39 and 46; below, 5120 rows 14.6 and 16.0 against 8.8 and 14.0, 5120 rows of 17408
+// inputs 23.0 and 24.5 against 17.6 and 23.5. Aligned weights are faster in the short-batch kernel at every size.
+constexpr uint32_t kInlineMinTiles = 8192;
 bool single_row_inline(const q4b_runtime *rt, uint64_t m, uint64_t k, const std::vector<Resolved> &jobs, uint32_t flags) {
     if (m != 1 || (flags & Q4B_FLAG_ACCUMULATE) || !rt->inline_max_halfs || k % 512 != 0 || k > rt->inline_max_halfs || k > q4k_stack_max_k()) return false;
     if (rt->rows_max_m == 0) return true;  // the short-batch kernel is switched off
     uint64_t tiles = 0;
     for (const Resolved &r : jobs) tiles += (r.n + 15u) / 16u;
-    return (tiles >= kInlineMinTiles || tiles < kInlineMaxTiles) && rows_byte_addressed(jobs.data(), (uint32_t)jobs.size(), (uint32_t)(k / 64));
+    return tiles >= kInlineMinTiles && rows_byte_addressed(jobs.data(), (uint32_t)jobs.size(), (uint32_t)(k / 64));
 }
 
 int profile_open(q4b_runtime *rt, cudaStream_t stream) {

@@ -113,3 +113,21 @@ def test_a_large_input_with_zero_weight_costs_its_neighbours_little(runtime, ora
     ref = oracle.matmul_f64(x, *trip, n)
     for r in range(m):
         assert oracle.rel_l2(out[r], ref[r]) <= 1e-5, r
+
+
+@pytest.mark.parametrize("n", [40, 5120, 16368, 16400])
+@pytest.mark.parametrize("offset", [0, 2])
+def test_single_rows_take_one_kernel_up_to_lm_head(runtime, oracle, n, offset):
+    """A plain single row takes the kernel that the residual form takes, so both give the same bits, and neither size nor offset
+    changes how its inputs are held (bar: as above, 1e-5 with one input of 1e4 and a weight of zero beside it)."""
+    k = 512
+    trip = _zero_weight_at(oracle.synth_q4(SEED, 92, n, k), 37)
+    job = upload_matrix(runtime, *trip, offset=offset)
+    x = np.random.default_rng(n).standard_normal((1, k)).astype(np.float32)
+    x[0, 37] = 1e4
+    bits = oracle.f32_to_bf16(x.reshape(-1))
+    for given, held in ((x.reshape(-1), x), (bits, oracle.bf16_to_f32(bits).reshape(1, k))):
+        out = runtime.q4_affine_matvec_mapped_batch(given, [job])[0]
+        added = runtime.q4_affine_matmul_add_mapped_batch(given, 1, [job], [np.zeros((1, n), dtype=np.float32)])[0]
+        assert np.array_equal(out, added.reshape(-1))
+        assert oracle.rel_l2(out, oracle.matmul_f64(held, *trip, n)) <= 1e-5

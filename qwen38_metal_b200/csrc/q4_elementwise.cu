@@ -2,19 +2,24 @@
 // weightless RMS-norm of the synthetic decode stack. Counterparts in the reference:
 // qwen38_swiglu_rows (shaders/qwen38.metal:4188-4198), qwen38_argmax_rows (:4201-4245),
 // qwen38_f32_to_f16 / qwen38_f16_to_f32 (:4166-4186), qwen38_rms_norm (:4250-4311).
+//
+// SwiGLU, argmax and RMS-norm are programmatic dependents like the projections they stand between, so that a projection behind one of them
+// requests its first weights while the one in front still runs. Launched the ordinary way they took that away: nine
+// projections and a SwiGLU 46.1 us against 38.8 for the projections alone. Their inputs are read through L2 and after the wait: a
+// read-only (non-coherent) load of a pointer that promises not to alias may be moved up, or hit a line cached before it.
 #include "q4_kernels.h"
 
 #include "q4_device.cuh"
 
 namespace q4 {
 
-__global__ void __launch_bounds__(256) swiglu_kernel(const float *__restrict__ gate, const float *__restrict__ up,
-                                                     uint64_t count, float *__restrict__ out_f32,
-                                                     uint16_t *__restrict__ out_bf16) {
+__global__ void __launch_bounds__(256) swiglu_kernel(const float *gate, const float *up, uint64_t count, float *out_f32, uint16_t *out_bf16) {
+    grid_dependency_wait();
+    grid_dependents_launch();
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
-    float g = gate[i];
-    float h = (g * (1.0f / (1.0f + expf(-g)))) * up[i];
+    float g = __ldcg(gate + i);
+    float h = (g * (1.0f / (1.0f + expf(-g)))) * __ldcg(up + i);
     if (out_f32) out_f32[i] = h;
     if (out_bf16) out_bf16[i] = (uint16_t)float_to_bf16_bits(h);
 }
@@ -60,14 +65,14 @@ __device__ __forceinline__ void argmax_block_reduce(float &bv, uint32_t &bi) {
 }
 
 // stage 1: grid (parts, m). stage 2: grid (1, m) over the `parts` partial pairs.
-__global__ void __launch_bounds__(256) argmax_partial_kernel(const float *__restrict__ logits, uint32_t n,
-                                                             uint32_t parts, float *__restrict__ pv,
-                                                             uint32_t *__restrict__ pi) {
+__global__ void __launch_bounds__(256) argmax_partial_kernel(const float *logits, uint32_t n, uint32_t parts, float *pv, uint32_t *pi) {
     const uint32_t row = blockIdx.y;
+    grid_dependency_wait();
+    grid_dependents_launch();
     const float *src = logits + (uint64_t)row * n;
     float bv = -INFINITY;
     uint32_t bi = 0xffffffffu;
-    for (uint32_t i = blockIdx.x * 256u + threadIdx.x; i < n; i += parts * 256u) argmax_merge(bv, bi, src[i], i);
+    for (uint32_t i = blockIdx.x * 256u + threadIdx.x; i < n; i += parts * 256u) argmax_merge(bv, bi, __ldcg(src + i), i);
     argmax_block_reduce(bv, bi);
     if (threadIdx.x == 0) {
         pv[row * parts + blockIdx.x] = bv;
@@ -75,13 +80,14 @@ __global__ void __launch_bounds__(256) argmax_partial_kernel(const float *__rest
     }
 }
 
-__global__ void __launch_bounds__(256) argmax_final_kernel(const float *__restrict__ pv, const uint32_t *__restrict__ pi,
-                                                           uint32_t parts, uint32_t index_base,
-                                                           uint32_t *__restrict__ tokens, float *__restrict__ values) {
+__global__ void __launch_bounds__(256) argmax_final_kernel(const float *pv, const uint32_t *pi, uint32_t parts, uint32_t index_base,
+                                                           uint32_t *tokens, float *values) {
+    grid_dependency_wait();
+    grid_dependents_launch();
     const uint32_t row = blockIdx.x;
     float bv = -INFINITY;
     uint32_t bi = 0xffffffffu;
-    for (uint32_t i = threadIdx.x; i < parts; i += 256u) argmax_merge(bv, bi, pv[row * parts + i], pi[row * parts + i]);
+    for (uint32_t i = threadIdx.x; i < parts; i += 256u) argmax_merge(bv, bi, __ldcg(pv + row * parts + i), __ldcg(pi + row * parts + i));
     argmax_block_reduce(bv, bi);
     if (threadIdx.x == 0) {
         // an all-NaN / empty row keeps the reference's starting index 0
@@ -92,12 +98,16 @@ __global__ void __launch_bounds__(256) argmax_final_kernel(const float *__restri
 
 // y = bf16(d / sqrt(mean(d^2) + eps)) for one vector per block; used by the synthetic stack to
 // keep the activation scale near one from layer to layer.
-__global__ void __launch_bounds__(1024) rms_unit_bf16_kernel(const float *__restrict__ in, uint32_t n, float eps,
-                                                            uint16_t *__restrict__ out) {
+__global__ void __launch_bounds__(1024) rms_unit_bf16_kernel(const float *in, uint32_t n, float eps, uint16_t *out) {
     __shared__ float warp_sums[32];
+    grid_dependency_wait();
+    grid_dependents_launch();
     const float *src = in + (uint64_t)blockIdx.x * n;
     float s = 0.f;
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) s += src[i] * src[i];
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+        const float v = __ldcg(src + i);
+        s += v * v;
+    }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
     if ((threadIdx.x & 31u) == 0) warp_sums[threadIdx.x >> 5] = s;
@@ -111,7 +121,7 @@ __global__ void __launch_bounds__(1024) rms_unit_bf16_kernel(const float *__rest
     __syncthreads();
     const float inv = rsqrtf(warp_sums[0] / (float)n + eps);
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x)
-        out[(uint64_t)blockIdx.x * n + i] = (uint16_t)float_to_bf16_bits(src[i] * inv);
+        out[(uint64_t)blockIdx.x * n + i] = (uint16_t)float_to_bf16_bits(__ldcg(src + i) * inv);
 }
 
 // dequantized_row (src/native.rs:4944-4987): out[i] = q*scale + bias for one row, byte-addressed
@@ -139,8 +149,7 @@ extern "C" cudaError_t q4k_dequantize_row(const uint8_t *w, const uint8_t *s, co
 
 extern "C" cudaError_t q4k_swiglu(const float *gate, const float *up, uint64_t count, float *out_f32,
                                   uint16_t *out_bf16, cudaStream_t stream) {
-    q4::swiglu_kernel<<<(uint32_t)((count + 255) / 256), 256, 0, stream>>>(gate, up, count, out_f32, out_bf16);
-    return cudaGetLastError();
+    return q4::launch_dependent(q4::swiglu_kernel, dim3((uint32_t)((count + 255) / 256)), 256, 0, stream, gate, up, count, out_f32, out_bf16);
 }
 
 extern "C" cudaError_t q4k_f32_to_bf16(const float *in, uint64_t count, uint16_t *out, cudaStream_t stream) {
@@ -156,13 +165,12 @@ extern "C" uint32_t q4k_argmax_parts(uint32_t n) {
 extern "C" cudaError_t q4k_argmax_rows(const float *logits, uint32_t m, uint32_t n, uint32_t index_base, float *pv,
                                        uint32_t *pi, uint32_t *tokens, float *values, cudaStream_t stream) {
     uint32_t parts = q4k_argmax_parts(n);
-    q4::argmax_partial_kernel<<<dim3(parts, m), 256, 0, stream>>>(logits, n, parts, pv, pi);
-    q4::argmax_final_kernel<<<m, 256, 0, stream>>>(pv, pi, parts, index_base, tokens, values);
-    return cudaGetLastError();
+    const cudaError_t e = q4::launch_dependent(q4::argmax_partial_kernel, dim3(parts, m), 256, 0, stream, logits, n, parts, pv, pi);
+    if (e != cudaSuccess) return e;
+    return q4::launch_dependent(q4::argmax_final_kernel, dim3(m), 256, 0, stream, pv, pi, parts, index_base, tokens, values);
 }
 
 extern "C" cudaError_t q4k_rms_unit_bf16(const float *in, uint32_t rows, uint32_t n, float eps, uint16_t *out,
                                          cudaStream_t stream) {
-    q4::rms_unit_bf16_kernel<<<rows, 1024, 0, stream>>>(in, n, eps, out);
-    return cudaGetLastError();
+    return q4::launch_dependent(q4::rms_unit_bf16_kernel, dim3(rows), 1024, 0, stream, in, n, eps, out);
 }

@@ -43,7 +43,6 @@
 
 #include <algorithm>
 #include <cstring>
-#include <utility>
 
 #include "q4_decomp.h"
 #include "q4_kernels.h"
@@ -890,28 +889,11 @@ bool encode_activation_map(EncodeTiledFn encode, CUtensorMap *map, const uint16_
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// a launch that may start while the kernel before it in the stream drains (both kernels wait before they touch its results)
-template <typename... Params, typename... Args>
-cudaError_t launch_dependent(void (*kernel)(Params...), uint32_t grid, uint32_t block, size_t smem, cudaStream_t stream, Args &&...args) {
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof cfg);
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
-}
-
 }  // namespace
 
 extern "C" cudaError_t q4k_gemm_prepare_x(const void *x, int x_is_f32, uint64_t elements, uint16_t *xp, cudaStream_t stream) {
     const uint64_t blocks = elements / 8;
-    return launch_dependent(q4::q4_gemm_prepare_x_kernel, (uint32_t)((blocks + 255) / 256), 256, 0, stream, x, x_is_f32, blocks, xp);
+    return q4::launch_dependent(q4::q4_gemm_prepare_x_kernel, dim3((uint32_t)((blocks + 255) / 256)), 256, 0, stream, x, x_is_f32, blocks, xp);
 }
 
 // xp: prepared activations [m][k] bf16 (q4k_gemm_prepare_x), 16-byte aligned. Up to kMaxJobs projections in one launch,
@@ -972,7 +954,7 @@ extern "C" cudaError_t q4k_gemm_tc(const Q4GemmPlan *plan, const uint16_t *xp, u
     if (p.stages > q4::kMaxStages || p.stages * p.bn > 1024u) return cudaErrorInvalidValue;  // (activation ring: at most four stages of 256 rows)
     const cudaError_t e = cudaFuncSetAttribute(q4::q4_gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)q4::kGemmSmemBytes);
     if (e != cudaSuccess) return e;
-    return launch_dependent(q4::q4_gemm_tc_kernel, 2u * p.workers, q4::kGemmThreads, q4::kGemmSmemBytes, stream, p);
+    return q4::launch_dependent(q4::q4_gemm_tc_kernel, dim3(2u * p.workers), q4::kGemmThreads, q4::kGemmSmemBytes, stream, p);
 }
 
 // 1 when the gate and up tensors can share one pair launch: the staged weight tiles of a projection have one geometry, so

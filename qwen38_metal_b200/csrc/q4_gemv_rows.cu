@@ -620,17 +620,7 @@ template <int NB, bool DC, bool MIS, int D>
 static cudaError_t rows_launch(const q4::RowsParams &p, uint32_t grid, size_t smem, cudaStream_t stream) {
     const cudaError_t e = cudaFuncSetAttribute(q4::q4_rows_kernel<NB, DC, MIS, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(q4::kRowsWarps * 32);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, q4::q4_rows_kernel<NB, DC, MIS, D>, p);
+    return q4::launch_dependent(q4::q4_rows_kernel<NB, DC, MIS, D>, dim3(grid), q4::kRowsWarps * 32, smem, stream, p);
 }
 
 extern "C" cudaError_t q4k_rows(const q4::RowsParams *params, uint32_t sm_count, cudaStream_t stream) {

@@ -128,6 +128,9 @@ int q4b_shard_read(q4b_runtime *rt, uint32_t shard_id, uint64_t offset, void *ho
 int q4b_shard_free(q4b_runtime *rt, uint32_t shard_id);
 /* MappedWeightBuffers::shard_count, src/metal_runtime.rs:624-626 */
 int q4b_shard_count(q4b_runtime *rt, uint32_t *count);
+/* Size and device address of a shard. Calls normally request weights while the kernel in front of them on the stream is
+ * still running; once the address of a shard has been asked for (device_ptr not null), calls that use the shard wait first, so
+ * that a kernel of the caller may write it like any other buffer. Ask before capturing calls in a graph. */
 int q4b_shard_info(q4b_runtime *rt, uint32_t shard_id, void **device_ptr, uint64_t *bytes);
 /* MappedWeightBuffers::offset_is_aligned, src/metal_runtime.rs:628-638, on the device address.
  * *aligned is 0 or 1. */

@@ -540,7 +540,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) q4_
             }
         }
     } else if (warp == 2) {
-        // ---- TMA producer: packed weights (they depend on nothing the kernel before this one wrote) ----
+        // ---- TMA producer: packed weights. They are requested (and parameters read) before this kernel's wait: the kernel in
+        // front is always the preparation or another GEMM of the same call, which writes no weights and lets this one start
+        // only after its own wait, when everything before the call is complete ----
         Ring ring;
         bool ok = true;
         while (ok && walk.next(p)) {

@@ -40,8 +40,8 @@
 // funnel shift, and the last words of a chunk lie in the first window of the next one, which is the next ring stage.
 // The instance without MIS keeps the shorter loop for launches whose tensors are all aligned.
 //
-// Launches are programmatic dependents of whatever runs in front of them: a block requests its first weights -- which no
-// kernel that lets a dependent start early ever writes -- and only then waits for the kernel before it.
+// Launches are programmatic dependents of whatever runs in front of them: a block requests its first weights and only then waits
+// for the kernel before it, unless that kernel may write them (weights_ahead: the caller holds the address of a shard).
 // What bounds it and what was measured (B200, a graph of calls, one call; in brackets the ring of single chunks with a rolled
 // loop, which issued 162 warp instructions a chunk where 100 will do): 4 rows x 34816 x 5120 24.3 us = 4.1 TB/s (26.0), 4 rows x
 // 248320 x 5120 129 us = 5.5 TB/s (147), 8 fp32 rows x 8192 x 5120 at a byte offset 17.7 us (18.5), one fp32 row x 5120 x 17408 at a
@@ -211,7 +211,8 @@ __global__ void __launch_bounds__(kRowsWarps * 32, 1) q4_rows_kernel(const __gri
     if (tr) tr[0] = rows_ns();
     bool first_run = true;
 
-    // weights do not depend on the kernel in front of this one, activation, output and scratch do
+    // activation, output and scratch depend on the kernel in front of this one, and weights the caller may write
+    if (!p.weights_ahead) grid_dependency_wait();
     request_quad(0);
     request_quad(1);
     grid_dependency_wait();

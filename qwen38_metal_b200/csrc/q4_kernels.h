@@ -79,6 +79,7 @@ struct RowsParams {
     uint32_t run;          // quads of chunks per warp (q4_rows_run)
     uint32_t part_slots;   // most contributions a part makes to one tile (q4_rows_part_slots)
     uint32_t accumulate;
+    uint32_t weights_ahead;  // weights may be requested before the kernel in front has finished
     uint32_t byte_addressed;  // some tensor misses a 16-byte boundary, or K % 512 != 0
     float *partials;       // [parts][part_slots][padded rows][tiles * 16] fp32, for tiles with several contributions
     unsigned int *counters;  // [tiles], zero between launches

@@ -112,6 +112,7 @@ struct HostPool {
 struct Shard {
     uint8_t *ptr = nullptr;
     uint64_t bytes = 0;
+    bool exposed = false;  // q4b_shard_info has given its address to the caller, whose kernels may write it
 };
 
 constexpr uint64_t kShardTailPad = 1024;  // prefetch and the unaligned window load may read a little past a tensor
@@ -119,6 +120,7 @@ constexpr uint64_t kShardTailPad = 1024;  // prefetch and the unaligned window l
 struct Resolved {
     const uint8_t *w, *s, *b;
     uint32_t n;
+    bool exposed;  // one of its shards is
 };
 
 }  // namespace
@@ -223,6 +225,7 @@ int resolve_job(q4b_runtime *rt, const q4b_job &job, uint64_t k, Resolved *out) 
     out->s = ss.ptr + job.scale_offset;
     out->b = bs.ptr + job.bias_offset;
     out->n = (uint32_t)job.output_rows;
+    out->exposed = ws.exposed || ss.exposed || bs.exposed;
     return Q4B_OK;
 }
 
@@ -264,6 +267,16 @@ bool single_row_inline(const q4b_runtime *rt, uint64_t m, uint64_t k, const std:
     uint64_t tiles = 0;
     for (const Resolved &r : jobs) tiles += (r.n + 15u) / 16u;
     return tiles >= kInlineMinTiles && rows_byte_addressed(jobs.data(), (uint32_t)jobs.size(), (uint32_t)(k / 64));
+}
+
+// Whether a short-batch launch may request weights before the kernel in front of it has finished. That kernel may be the caller's
+// own: it can write a shard only if the caller has the shard's address, and the launch is not ordered behind its writes if it
+// lets dependents start early (nor, by the letter, before the wait if it does not). What this library writes into shards is
+// complete before the writing call returns.
+bool rows_weights_ahead(const Resolved *jobs, uint32_t n_jobs) {
+    for (uint32_t i = 0; i < n_jobs; ++i)
+        if (jobs[i].exposed) return false;
+    return true;
 }
 
 int profile_open(q4b_runtime *rt, cudaStream_t stream) {
@@ -540,6 +553,7 @@ int launch_rows(q4b_runtime *rt, const void *x_dev, int x_dtype, uint32_t m, uin
     p.part_chunks = part_chunks;
     p.tiles = tiles;
     p.accumulate = (flags & Q4B_FLAG_ACCUMULATE) ? 1u : 0u;
+    p.weights_ahead = rows_weights_ahead(jobs, n_jobs) ? 1u : 0u;
     p.run = q4_rows_run(tiles, part_chunks, parts, (uint32_t)rt->sm_count);
     p.part_slots = q4_rows_part_slots(p.cpt, parts, p.run);
     if (parts > 1 || p.part_slots > 1) {
@@ -991,7 +1005,10 @@ extern "C" int q4b_shard_info(q4b_runtime *rt, uint32_t shard_id, void **device_
     if (int st = check_rt(rt)) return st;
     std::lock_guard<std::recursive_mutex> lock(rt->mu);
     if (int st = shard_range(rt, shard_id, 0, 0)) return st;
-    if (device_ptr) *device_ptr = rt->shards[shard_id].ptr;
+    if (device_ptr) {
+        *device_ptr = rt->shards[shard_id].ptr;
+        rt->shards[shard_id].exposed = true;
+    }
     if (bytes) *bytes = rt->shards[shard_id].bytes;
     return Q4B_OK;
 }
@@ -1970,8 +1987,8 @@ extern "C" int q4b_describe_dispatch(q4b_runtime *rt, int x_dtype, uint64_t m, u
         const uint32_t mb = (uint32_t)std::min<uint64_t>(m, std::min(rt->rows_max_m, q4k_rows_per_launch(mis)));
         const uint32_t parts = q4k_rows_plan(mb, (uint32_t)k, tiles, (uint32_t)rt->sm_count, mis, f32, &part_chunks);
         if (parts) {
-            snprintf(text, text_len, "rows_i8 (short batch, integer tensor cores) rows_per_launch=%u k_parts=%u chunks_per_part=%u jobs=%u (a 16-byte aligned activation is assumed)",
-                     mb, parts, part_chunks, n_jobs);
+            snprintf(text, text_len, "rows_i8 (short batch, integer tensor cores) rows_per_launch=%u k_parts=%u chunks_per_part=%u jobs=%u weights_ahead=%d (a 16-byte aligned activation is assumed)",
+                     mb, parts, part_chunks, n_jobs, rows_weights_ahead(resolved.data(), n_jobs) ? 1 : 0);
             return Q4B_OK;
         }
     }

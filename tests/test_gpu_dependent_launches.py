@@ -73,3 +73,40 @@ def test_a_row_of_calls_reads_what_the_call_before_wrote(runtime, m, captured):
         runtime.device_status()
         for got, ref in zip(seen + [tokens, values], expected):
             assert torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("m,offset", [(1, 0), (1, 2), (4, 0), (8, 2)])
+def test_calls_wait_for_weights_that_the_caller_can_write(runtime, m, offset):
+    """Asking for a shard's address makes the calls that use it wait for the kernel in front before they read weights. A copy of
+    the caller's into the shard, directly in front of the call, is what the call computes with."""
+    import torch
+
+    from qwen38_metal_b200 import capi
+
+    n, k = 512, 1024
+    job, other = _job(runtime, 20, n, k, offset), _job(runtime, 21, n, k, offset)
+    x = torch.randn(m, k, generator=torch.Generator(device="cuda").manual_seed(m), device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+
+    def call(j):
+        out = torch.zeros(m, n, device="cuda")
+        runtime.matmul_batch_device(x.data_ptr(), capi.Q4B_F32, m, k, [j], [out.data_ptr()], 0, stream)
+        return out
+
+    first, second = call(job), call(other)
+    assert "weights_ahead=1" in runtime.describe_dispatch(capi.Q4B_F32, m, k, [job])
+    fresh = [torch.from_numpy(runtime.read_shard(b, 0, b.length)).cuda() for b in (other.weights, other.scales, other.biases)]
+    torch.cuda.synchronize()
+
+    class Raw:  # a shard as torch sees memory
+        def __init__(self, buf):
+            self.__cuda_array_interface__ = {"shape": (buf.length,), "typestr": "|u1", "data": (runtime.shard_pointer(buf), False), "version": 3}
+
+    shards = [torch.as_tensor(Raw(b), device="cuda") for b in (job.weights, job.scales, job.biases)]
+    for s, f in zip(shards, fresh):
+        torch.add(f, 0, out=s)  # a kernel, not a copy
+    again = call(job)
+    runtime.device_status()
+    assert "weights_ahead=0" in runtime.describe_dispatch(capi.Q4B_F32, m, k, [job])
+    assert "weights_ahead=1" in runtime.describe_dispatch(capi.Q4B_F32, m, k, [other])
+    assert torch.equal(again, second) and not torch.equal(first, second)

@@ -139,6 +139,11 @@ struct Q4GemmPlan {
     uint32_t counters;
 };
 
+// The most scratch any plan asks for: two parts of a 256 x 256 tile per worker, and a counter per warp's share of the tiles left
+// over after the whole rounds, of which there are fewer than two per worker.
+inline uint64_t q4_gemm_most_partial_floats(uint32_t pairs) { return (uint64_t)pairs * 2u * 256u * 256u; }
+inline uint32_t q4_gemm_most_counters(uint32_t pairs) { return (2u * pairs - 1u) * 8u; }
+
 // row tiles of an n-row projection: 256 weight rows of one tensor, or (pair mode) 128 gate rows and the same up rows
 Q4_HD uint32_t q4_gemm_row_tiles(uint32_t n, uint32_t pair) { return pair ? (n + 127u) / 128u : (n + 255u) / 256u; }
 

@@ -65,10 +65,11 @@ struct Pool {
     size_t capacity = 0;
     void *outgrown[64];  // (at most one per power of two)
     int n_outgrown = 0;
-    cudaError_t ensure(size_t bytes) {
+    cudaError_t ensure(size_t bytes, bool exact = false) {
         if (bytes <= capacity) return cudaSuccess;
         size_t want = 256;
         while (want < bytes) want <<= 1;
+        if (exact) want = bytes;  // (what it needs is known: it will not grow)
         void *fresh = nullptr;
         cudaError_t e = cudaMalloc(&fresh, want);
         if (e != cudaSuccess) return e;
@@ -480,11 +481,10 @@ int launch_gemm(q4b_runtime *rt, const uint16_t *xp, uint32_t m, uint32_t k, con
     Q4GemmPlan plan;
     q4_gemm_plan(m, k, row_tiles, (uint32_t)rt->sm_count / 2u, &plan);
     if (plan.counters) {
-        Q4B_CUDA(rt->gemm_parts.ensure(plan.partial_floats * 4), "partial tile scratch");
-        const size_t had = rt->gemm_counters.capacity;
-        Q4B_CUDA(rt->gemm_counters.ensure((size_t)plan.counters * 4), "tile counter scratch");
-        // (put back to zero by the kernel itself, like the short-batch kernel's)
-        if (rt->gemm_counters.capacity != had || rt->gemm_failures_seen != rt->failures) {
+        if (plan.partial_floats * 4 > rt->gemm_parts.capacity || (size_t)plan.counters * 4 > rt->gemm_counters.capacity)
+            return fail(Q4B_UNSUPPORTED, "launch plan exceeds the scratch set aside for it");
+        // (the counters are put back to zero by the kernel itself, like the short-batch kernel's)
+        if (rt->gemm_failures_seen != rt->failures) {
             Q4B_CUDA(cudaMemsetAsync(rt->gemm_counters.ptr, 0, rt->gemm_counters.capacity, stream), "tile counter reset");
             rt->gemm_failures_seen = rt->failures;
         }
@@ -758,10 +758,18 @@ extern "C" int q4b_runtime_create(int device_ordinal, q4b_runtime **out) {
     if (e == cudaSuccess) e = rt->error_flag.ensure(256);
     if (e == cudaSuccess) e = cudaMemset(rt->error_flag.ptr, 0, rt->error_flag.capacity);
     if (e == cudaSuccess) e = rt->status.ensure(sizeof(int));
-    // enough for lm_head of four rows, 248320 wide; larger launches grow it
-    if (e == cudaSuccess) e = rt->rows_partials.ensure((size_t)8 << 20);
+    // what a single row of up to 8192 inputs and 2^18 outputs needs at most (two parts, two contributions each), so that decode
+    // calls do not allocate; larger launches grow it
+    if (e == cudaSuccess) e = rt->rows_partials.ensure((size_t)2 * 2 * 2 * 16384 * 16 * 4);
     if (e == cudaSuccess) e = rt->rows_counters.ensure(16384 * 4);
     if (e == cudaSuccess) e = cudaMemset(rt->rows_counters.ptr, 0, rt->rows_counters.capacity);
+    // all that the tensor-core GEMM can ask for (39 MB on 148 SMs): grown on demand, most prompt calls allocated in their first pass
+    // (gate+up of 512 rows 0.57 ms without that, 0.9 with it)
+    if (e == cudaSuccess) e = rt->gemm_parts.ensure(q4_gemm_most_partial_floats((uint32_t)rt->sm_count / 2u) * 4, true);
+    if (e == cudaSuccess) e = rt->gemm_counters.ensure((size_t)q4_gemm_most_counters((uint32_t)rt->sm_count / 2u) * 4);
+    if (e == cudaSuccess) e = cudaMemset(rt->gemm_counters.ptr, 0, rt->gemm_counters.capacity);
+    // (memsets return before they are done, and the runtime's stream does not wait for the default one)
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
     if (const char *unf = getenv("Q4B_MLP_UNFUSED")) rt->mlp_unfused = strtol(unf, nullptr, 10) != 0;
     if (const char *off = getenv("Q4B_NO_INLINE")) rt->inline_off = strtol(off, nullptr, 10) != 0;
     if (e == cudaSuccess && !rt->inline_off) {

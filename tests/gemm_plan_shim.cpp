@@ -10,6 +10,7 @@ extern "C" int shim_gemm_plan(uint32_t m, uint32_t k, uint32_t row_tiles, uint32
     Q4GemmPlan p;
     q4_gemm_plan(m, k, row_tiles, pairs, &p);
     const uint32_t ks = q4_gemm_k_stages(k);
+    if (p.partial_floats > q4_gemm_most_partial_floats(pairs) || p.counters > q4_gemm_most_counters(pairs)) return 8;
     if (p.bn % 32 || p.bn < 32 || p.bn > 256 || p.accs * p.bn + 64 * p.stages > 512 || p.stages < 4) return 1;
     if (p.tiles != row_tiles * p.tiles_m || p.tiles_m * p.bn < m || (p.tiles_m - 1) * p.bn >= m) return 2;
     if (p.workers == 0 || p.workers > pairs || p.tail_workers > p.workers) return 3;

@@ -78,3 +78,32 @@ def test_captured_call_survives_a_call_that_outgrows_its_scratch(small, large):
         assert all(np.isfinite(o.cpu().numpy()).all() and float(o.abs().sum()) > 0 for o in first)
     finally:
         rt.close()
+
+
+def test_first_calls_do_not_allocate():
+    """A single row never allocates, and of prompt rows only the converted activation does (once for all calls of its size): the
+    scratch for tiles cut between SM pairs is bounded and set aside with the runtime."""
+    import torch
+
+    from qwen38_metal_b200 import capi
+    from qwen38_metal_b200.runtime import CudaRuntime
+
+    rt = CudaRuntime(0)
+    stream = torch.cuda.current_stream().cuda_stream
+    try:
+        calls = []
+        for m, rows, k, offset in ((1, (5120,), 5120, 0), (1, (6144, 1024, 1024), 5120, 2), (600, (256,), 5120, 0), (600, (5000, 300), 5120, 2), (200, (19000,), 5120, 0)):
+            x = torch.randn(m, k, device="cuda").to(torch.bfloat16)
+            calls.append((x, m, k, _jobs(rt, rows, k, offset), [torch.zeros(m, n, device="cuda") for n in rows]))
+        free = []
+        for x, m, k, jobs, outs in calls:
+            torch.cuda.synchronize()
+            free.append(torch.cuda.mem_get_info()[0])
+            rt.matmul_batch_device(x.data_ptr(), capi.Q4B_BF16, m, k, jobs, [o.data_ptr() for o in outs], 0, stream)
+            rt.device_status()
+        free.append(torch.cuda.mem_get_info()[0])
+        assert free[0] == free[1] == free[2]  # single rows
+        assert 0 <= free[2] - free[3] <= 16 << 20  # 600 x 5120 bf16, rounded up
+        assert free[3] == free[4] == free[5]
+    finally:
+        rt.close()

@@ -52,6 +52,19 @@ def test_every_quad_once_and_shares_agree(shim, k, tiles, cap, mp, tw):
             assert len(seen[item]) <= slots
 
 
+@pytest.mark.parametrize("cap", [78, 48])  # aligned, byte-addressed
+def test_single_rows_fit_the_scratch_a_runtime_sets_aside(shim, cap):
+    """8 MB of partial sums (two padded rows, fp32) and 16384 tile counters hold any single row of up to 8192 inputs and 2^18
+    outputs, so that a decode call does not allocate."""
+    longest = C.c_uint32(0)
+    for k in (64, 512, 1600, 4096, 5120, 6144, 8192):
+        cpt = (k // 64 + 1) // 2
+        for tiles in list(range(1, 400)) + list(range(400, 16384, 97)) + [16384]:
+            parts = shim.shim_rows_plan_for(cpt, tiles, 148, cap, 1, 2, C.byref(longest))
+            slots = shim.shim_rows_part_slots(cpt, parts, shim.shim_rows_run(tiles, longest.value, parts, 148))
+            assert parts * slots * 2 * tiles * 64 <= 8 << 20, (k, tiles)
+
+
 def test_a_launch_with_more_quads_than_32_bits_is_refused(shim):
     longest = C.c_uint32(0)
     assert shim.shim_rows_plan_for(136, 0xFFFFFFF, 148, 92, 1, 2, C.byref(longest)) == 0

@@ -171,6 +171,8 @@ int q4b_dequantize_row(q4b_runtime *rt, const q4b_job *job, uint64_t k, uint64_t
 #define Q4B_FLAG_STREAM 2u     /* this call uses the streaming (decode) kernels whatever m is */
 #define Q4B_FLAG_TENSOR 4u     /* this call uses the tensor-core GEMM whatever m is */
 
+/* An output may lie over the activation, and projections of a call may share an output (they then write, or add, in the order
+ * given); such calls take more launches. */
 int q4b_matmul_batch_device(q4b_runtime *rt, const void *x_dev, int x_dtype, uint64_t m, uint64_t k,
                             const q4b_job *jobs, uint32_t n_jobs, float *const *outputs_dev, uint32_t flags,
                             void *stream);

@@ -270,6 +270,20 @@ bool single_row_inline(const q4b_runtime *rt, uint64_t m, uint64_t k, const std:
     return tiles >= kInlineMinTiles && rows_byte_addressed(jobs.data(), (uint32_t)jobs.size(), (uint32_t)(k / 64));
 }
 
+bool ranges_overlap(const void *a, size_t a_bytes, const void *b, size_t b_bytes) {
+    return (uintptr_t)a < (uintptr_t)b + b_bytes && (uintptr_t)b < (uintptr_t)a + a_bytes;
+}
+
+// Projections from number j0 on that one launch takes: at most kMaxJobs, and none whose output shares memory with that of an
+// earlier one. Projections that share an output (two added into one residual) run in the order given, in launches of their own.
+uint32_t launch_group(const std::vector<Resolved> &jobs, float *const *outs, uint64_t m, size_t j0) {
+    const size_t end = std::min(jobs.size(), j0 + (size_t)q4::kMaxJobs);
+    for (size_t j = j0 + 1; j < end; ++j)
+        for (size_t i = j0; i < j; ++i)
+            if (ranges_overlap(outs[i], (size_t)m * jobs[i].n * 4, outs[j], (size_t)m * jobs[j].n * 4)) return (uint32_t)(j - j0);
+    return (uint32_t)(end - j0);
+}
+
 // Whether a short-batch launch may request weights before the kernel in front of it has finished. That kernel may be the caller's
 // own: it can write a shard only if the caller has the shard's address, and the launch is not ordered behind its writes if it
 // lets dependents start early (nor, by the letter, before the wait if it does not). What this library writes into shards is
@@ -505,8 +519,9 @@ int enqueue_gemm(q4b_runtime *rt, const void *x_dev, int x_dtype, uint64_t m, ui
     Q4B_CUDA(q4k_gemm_prepare_x(x_dev, x_dtype == Q4B_F32 ? 1 : 0, m * k, (uint16_t *)rt->gemm_x.ptr, stream),
              "q4_gemm_prepare_x launch");
     rt->launches++;
-    for (size_t j0 = 0; j0 < jobs.size(); j0 += q4::kMaxJobs) {
-        const uint32_t nj = (uint32_t)std::min(jobs.size() - j0, (size_t)q4::kMaxJobs);
+    uint32_t nj = 0;
+    for (size_t j0 = 0; j0 < jobs.size(); j0 += nj) {
+        nj = launch_group(jobs, outs, m, j0);
         if (int st = launch_gemm(rt, (const uint16_t *)rt->gemm_x.ptr, (uint32_t)m, (uint32_t)k, &jobs[j0], nj, outs + j0, nullptr, 0, flags, stream))
             return st;
     }
@@ -591,10 +606,16 @@ int enqueue_matmul(q4b_runtime *rt, const void *x_dev, int x_dtype, uint64_t m, 
     // tensor-core kernel, as do single rows but for the few that the persistent kernel takes.
     bool rows = !want_tensor && (m >= 2 || (!single && m < rt->gemm_min_m)) && rt->rows_max_m >= 1 && (want_stream || m <= rt->rows_max_m) &&
                 ((uintptr_t)x_dev & 15u) == 0;
+    // A call that writes over its own activation: blocks of these kernels read it at different times, the streaming kernel (and the
+    // GEMM) from a copy.
+    bool in_place = false;
+    for (size_t j = 0; j < jobs.size(); ++j) in_place |= ranges_overlap(x_dev, (size_t)m * k * esize, outs[j], (size_t)m * jobs[j].n * 4);
+    rows &= !in_place;
     uint32_t rows_step = rt->rows_max_m;  // rows per launch
-    for (size_t j0 = 0; j0 < jobs.size() && rows; j0 += q4::kMaxJobs) {
+    uint32_t nj = 0;
+    for (size_t j0 = 0; j0 < jobs.size() && rows; j0 += nj) {
         uint32_t tiles = 0, part_chunks = 0;
-        const uint32_t nj = (uint32_t)std::min(jobs.size() - j0, (size_t)q4::kMaxJobs);
+        nj = launch_group(jobs, outs, m, j0);
         for (size_t j = j0; j < j0 + nj; ++j) tiles += (jobs[j].n + 15u) / 16u;
         const int mis = rows_byte_addressed(&jobs[j0], nj, (uint32_t)(k / 64)) ? 1 : 0;
         rows_step = std::min(rows_step, q4k_rows_per_launch(mis));
@@ -610,8 +631,8 @@ int enqueue_matmul(q4b_runtime *rt, const void *x_dev, int x_dtype, uint64_t m, 
         for (uint64_t m0 = 0; m0 < m; m0 += rows_step) {
             const uint32_t mb = (uint32_t)std::min<uint64_t>(m - m0, rows_step);
             const uint8_t *xb = (const uint8_t *)x_dev + m0 * k * esize;
-            for (size_t j0 = 0; j0 < jobs.size(); j0 += q4::kMaxJobs) {
-                const uint32_t nj = (uint32_t)((jobs.size() - j0) < (size_t)q4::kMaxJobs ? (jobs.size() - j0) : (size_t)q4::kMaxJobs);
+            for (size_t j0 = 0; j0 < jobs.size(); j0 += nj) {
+                nj = launch_group(jobs, outs, m, j0);
                 float *o[q4::kMaxJobs];
                 for (uint32_t i = 0; i < nj; ++i) o[i] = outs[j0 + i] + m0 * jobs[j0 + i].n;
                 const int st = launch_rows(rt, xb, x_dtype, mb, (uint32_t)k, &jobs[j0], nj, o, flags, stream);
@@ -622,9 +643,9 @@ int enqueue_matmul(q4b_runtime *rt, const void *x_dev, int x_dtype, uint64_t m, 
         return Q4B_OK;
     }
     if (want_tensor || (!want_stream && m >= rt->gemm_min_m)) return enqueue_gemm(rt, x_dev, x_dtype, m, k, jobs, outs, flags, stream);
-    if (single) {
-        for (size_t j0 = 0; j0 < jobs.size(); j0 += q4::kMaxJobs) {
-            const uint32_t nj = (uint32_t)((jobs.size() - j0) < (size_t)q4::kMaxJobs ? (jobs.size() - j0) : (size_t)q4::kMaxJobs);
+    if (single && !in_place) {
+        for (size_t j0 = 0; j0 < jobs.size(); j0 += nj) {
+            nj = launch_group(jobs, outs, m, j0);
             if (int st = launch_single_row(rt, x_dev, x_dtype, (uint32_t)k, &jobs[j0], nj, outs + j0, stream)) return st;
         }
         return Q4B_OK;
@@ -633,8 +654,8 @@ int enqueue_matmul(q4b_runtime *rt, const void *x_dev, int x_dtype, uint64_t m, 
     for (uint64_t m0 = 0; m0 < m; m0 += rows_per_launch) {
         const uint32_t mb = (uint32_t)((m - m0) < rows_per_launch ? (m - m0) : rows_per_launch);
         const uint8_t *xb = (const uint8_t *)x_dev + m0 * k * esize;
-        for (size_t j0 = 0; j0 < jobs.size(); j0 += q4::kMaxJobs) {
-            const uint32_t nj = (uint32_t)((jobs.size() - j0) < (size_t)q4::kMaxJobs ? (jobs.size() - j0) : (size_t)q4::kMaxJobs);
+        for (size_t j0 = 0; j0 < jobs.size(); j0 += nj) {
+            nj = launch_group(jobs, outs, m, j0);
             float *o[q4::kMaxJobs];
             for (uint32_t i = 0; i < nj; ++i) o[i] = outs[j0 + i] + m0 * jobs[j0 + i].n;
             int st = launch_streaming(rt, xb, x_dtype, mb, (uint32_t)k, &jobs[j0], nj, o, nullptr, flags, stream);

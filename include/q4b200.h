@@ -14,8 +14,9 @@
  *     return. They serialise on an internal lock, as the reference's pooled entry points do
  *     (Mutex<Q4ActivationPool>, src/metal_runtime.rs:3627-3630), so one runtime may be
  *     shared by several host threads;
- *   - `_device` twins take device pointers and a cudaStream_t (passed as void*), enqueue
- *     work and return without synchronising. They use the runtime's scratch buffers: calls
+ *   - `_device` twins take device pointers (activations 16-byte aligned, else
+ *     Q4B_INVALID_ARGUMENT) and a cudaStream_t (passed as void*), enqueue work and return
+ *     without synchronising. They use the runtime's scratch buffers: calls
  *     on one runtime must be ordered on the device (one stream, or events). Scratch grows on
  *     first use of a larger shape, so run a shape once before capturing it in a CUDA graph.
  *     Scratch that a later, larger call outgrows stays allocated until q4b_runtime_destroy, so

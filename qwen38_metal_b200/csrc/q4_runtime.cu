@@ -1078,6 +1078,7 @@ extern "C" int q4b_argmax_batch_device(q4b_runtime *rt, const void *x_dev, int x
     if (int st = check_rt(rt)) return st;
     if (int st = check_dtype(x_dtype)) return st;
     if (!x_dev || !tokens_dev || !job) return fail(Q4B_INVALID_ARGUMENT, "activation, job or token pointer is null");
+    if ((uintptr_t)x_dev & 15u) return fail(Q4B_INVALID_ARGUMENT, "device activations must be 16-byte aligned");
     std::lock_guard<std::recursive_mutex> lock(rt->mu);
     DeviceGuard guard(rt->device);
     std::vector<Resolved> resolved;
@@ -1214,6 +1215,7 @@ extern "C" int q4b_mlp_batch_device(q4b_runtime *rt, const void *x_dev, int x_dt
     if (int st = check_rt(rt)) return st;
     if (int st = check_dtype(x_dtype)) return st;
     if (!x_dev || !out_dev || !gate || !up || !down) return fail(Q4B_INVALID_ARGUMENT, "activation, job or output pointer is null");
+    if ((uintptr_t)x_dev & 15u) return fail(Q4B_INVALID_ARGUMENT, "device activations must be 16-byte aligned");
     if (m == 0 || k == 0) return fail(Q4B_EMPTY_DIMENSION, "matrix dimensions must be greater than zero");
     // gate and up must agree (src/metal_runtime.rs:4511-4517)
     if (gate->output_rows != up->output_rows)

@@ -123,3 +123,27 @@ def test_host_buffer_token_step(runtime, oracle):
     got_token, got_best = chain.run_host(x_bits)
     assert (got_token, got_best) == (token, best)
     chain.close()
+
+
+@pytest.mark.parametrize("m", [1, 4, 20])
+def test_misaligned_device_activations_are_refused(runtime, oracle, m):
+    """Every kernel reads activations 16 bytes at a time: all device entry points that take one refuse a pointer off that
+    boundary before anything is launched."""
+    import torch
+
+    from qwen38_metal_b200 import capi
+    from qwen38_metal_b200.runtime import Q4RuntimeError
+
+    k = 512
+    gate, up, down = (upload_matrix(runtime, *oracle.synth_q4(503, i, n, c)) for i, (n, c) in enumerate(((256, k), (256, k), (96, 256))))
+    x = torch.zeros(m * k + 8, dtype=torch.bfloat16, device="cuda")
+    out, tokens = torch.zeros(m * 256, device="cuda"), torch.zeros(m, dtype=torch.int32, device="cuda")
+    stream, at = torch.cuda.current_stream().cuda_stream, x.data_ptr() + 2
+    before = runtime.launch_count()
+    for call in (lambda: runtime.matmul_batch_device(at, capi.Q4B_BF16, m, k, [gate], [out.data_ptr()], 0, stream),
+                 lambda: runtime.argmax_batch_device(at, capi.Q4B_BF16, m, k, gate, 0, tokens.data_ptr(), 0, stream),
+                 lambda: runtime.mlp_batch_device(at, capi.Q4B_BF16, m, k, gate, up, down, out.data_ptr(), stream)):
+        with pytest.raises(Q4RuntimeError) as err:
+            call()
+        assert err.value.kind == "InvalidArgument"
+    assert runtime.launch_count() == before

@@ -72,18 +72,18 @@ Q4_HD uint32_t q4_rows_part_begin(uint32_t cpt, uint32_t parts, uint32_t part) {
     return c < cpt ? c : cpt;
 }
 
-// Inside a part the quads (four chunks) of all items -- an item is a 16-row tile, or two -- are numbered item-major and
-// every warp of the part's blocks takes `run` consecutive ones. Contributions (warps) of a part with `quads` quads per
-// item to item `item`; warp item * quads / run makes the first.
-Q4_HD uint32_t q4_rows_shares(uint32_t item, uint32_t quads, uint32_t run) { return (item * quads + quads - 1u) / run - item * quads / run + 1u; }
+// Inside a part the quads (four chunks) of all 16-row tiles are numbered tile-major and every warp of the part's blocks
+// takes `run` consecutive ones. Contributions (warps) of a part with `quads` quads per tile to tile `tile`; warp
+// tile * quads / run makes the first.
+Q4_HD uint32_t q4_rows_shares(uint32_t tile, uint32_t quads, uint32_t run) { return (tile * quads + quads - 1u) / run - tile * quads / run + 1u; }
 
 // quads a warp takes: the longest part's, spread over its warps
-Q4_HD uint32_t q4_rows_run(uint32_t items, uint32_t part_chunks, uint32_t parts, uint32_t sm_count) {
+Q4_HD uint32_t q4_rows_run(uint32_t tiles, uint32_t part_chunks, uint32_t parts, uint32_t sm_count) {
     const uint32_t warps = sm_count / parts * 16u;
-    return (items * ((part_chunks + 3u) / 4u) + warps - 1u) / warps;
+    return (tiles * ((part_chunks + 3u) / 4u) + warps - 1u) / warps;
 }
 
-// the most contributions any part makes to one item
+// the most contributions any part makes to one tile
 inline uint32_t q4_rows_part_slots(uint32_t cpt, uint32_t parts, uint32_t run) {
     uint32_t most = 1;
     for (uint32_t p = 0; p < parts; ++p) {
@@ -94,26 +94,25 @@ inline uint32_t q4_rows_part_slots(uint32_t cpt, uint32_t parts, uint32_t run) {
     return most;
 }
 
-// How many parts to cut K into for `tiles` 16-row tiles on `sm_count` SMs of 16 warps, each warp walking `tw` tiles at
-// a time, when a block can hold at most `cap` chunks of activation digits of `mp` rows; 0 when no split fits.
+// How many parts to cut K into for `tiles` 16-row tiles on `sm_count` SMs of 16 warps, when a block can hold at most `cap`
+// chunks of activation digits of `mp` rows; 0 when no split fits.
 // *part_chunks: chunks of the longest part; *cost_out: the estimate the choice was made by.
-// Cost of a split in chunk times: the chunks of a warp's run (a chunk of two tiles costs 1.75, measured; the activation's
-// fragments are read once for both), about three more for a tile it finishes alone and six for one whose sums meet in
-// scratch, and the conversion of the part's activation before the first chunk.
-Q4_HD uint32_t q4_rows_plan(uint32_t cpt, uint32_t tiles, uint32_t sm_count, uint32_t cap, uint32_t tw, uint32_t mp, uint32_t *part_chunks, double *cost_out) {
-    if (cpt == 0 || tiles == 0 || sm_count == 0 || tw == 0) return 0;
-    const uint32_t all = (cpt + 3u) / 4u, items = (tiles + tw - 1u) / tw;
-    if ((uint64_t)items * all + (uint64_t)all * 65536u > 0xffffffffull) return 0;  // quads are counted in 32 bits
+// Cost of a split in chunk times: the chunks of a warp's run, about three more for a tile it finishes alone and six for one
+// whose sums meet in scratch, and the conversion of the part's activation before the first chunk.
+Q4_HD uint32_t q4_rows_plan(uint32_t cpt, uint32_t tiles, uint32_t sm_count, uint32_t cap, uint32_t mp, uint32_t *part_chunks, double *cost_out) {
+    if (cpt == 0 || tiles == 0 || sm_count == 0) return 0;
+    const uint32_t all = (cpt + 3u) / 4u;
+    if ((uint64_t)tiles * all + (uint64_t)all * 65536u > 0xffffffffull) return 0;  // quads are counted in 32 bits
     uint32_t best = 0;
     double best_cost = 0.0;
     for (uint32_t parts = 1; parts <= all && parts <= sm_count && parts <= 32u; ++parts) {
         const uint32_t quads = (all + parts - 1u) / parts;
         if (quads * 4u > cap && !(parts == 1u && cpt <= cap)) continue;
-        const uint32_t run = q4_rows_run(items, quads * 4u, parts, sm_count);
+        const uint32_t run = q4_rows_run(tiles, quads * 4u, parts, sm_count);
         const bool split = run % quads != 0;
         const uint32_t pieces = (run + quads - 1u) / quads + (split && quads % run != 0 ? 1u : 0u);
         const double piece = parts == 1u ? 3.0 : 6.0;
-        const double cost = 4.0 * run * (tw == 1u ? 1.0 : 1.75) + pieces * piece + (split ? 6.0 : 0.0) + 0.02 * mp * quads * 4.0 + 0.3 * parts;
+        const double cost = 4.0 * run + pieces * piece + (split ? 6.0 : 0.0) + 0.02 * mp * quads * 4.0 + 0.3 * parts;
         if (best == 0 || cost < best_cost * 0.98) {
             best_cost = cost;
             best = parts;

@@ -612,7 +612,7 @@ extern "C" uint32_t q4k_rows_plan(uint32_t m, uint32_t k, uint32_t tiles, uint32
     if (m < 1 || m > q4k_rows_per_launch(mis) || k == 0 || k % (mis ? 64u : 512u) != 0 || tiles == 0) return 0;
     const uint32_t mp = q4::rows_padded(m);
     const uint32_t cap = rows_part_capacity(mp, mis != 0, q4::rows_dc(m), q4::rows_digits(m, mis != 0, f32 != 0));
-    return cap ? q4_rows_plan((k / 64u + 1u) / 2u, tiles, sm_count, cap, 1u, mp, part_chunks, nullptr) : 0u;
+    return cap ? q4_rows_plan((k / 64u + 1u) / 2u, tiles, sm_count, cap, mp, part_chunks, nullptr) : 0u;
 }
 
 extern "C" uint32_t q4k_rows_padded(uint32_t m) { return q4::rows_padded(m); }

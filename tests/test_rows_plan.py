@@ -1,5 +1,5 @@
 """The short-batch kernel's cut of a launch into runs of quads (csrc/q4_decomp.h), followed on the CPU: every quad of every
-item is taken by exactly one warp, and what a warp that finishes a shared item expects -- how many contributions, in
+tile is taken by exactly one warp, and what a warp that finishes a shared tile expects -- how many contributions, in
 which scratch slots -- is what the other warps do."""
 import ctypes as C
 import os
@@ -20,15 +20,14 @@ def shim(tmp_path_factory):
 
 @pytest.mark.parametrize("k", [64, 192, 512, 1600, 5120, 5184, 17408])
 @pytest.mark.parametrize("tiles", [1, 3, 64, 320, 533, 2176, 15520])
-@pytest.mark.parametrize("cap,mp,tw", [(92, 2, 1), (31, 4, 1), (16, 8, 1), (21, 8, 2), (8, 16, 1)])
-def test_every_quad_once_and_shares_agree(shim, k, tiles, cap, mp, tw):
+@pytest.mark.parametrize("cap,mp", [(102, 2), (78, 2), (48, 2), (51, 4), (24, 4), (26, 8), (12, 8), (13, 16)])  # what a block holds
+def test_every_quad_once_and_shares_agree(shim, k, tiles, cap, mp):
     sms = 148
     cpt = (k // 64 + 1) // 2
     longest = C.c_uint32(0)
-    parts = shim.shim_rows_plan_for(cpt, tiles, sms, cap, tw, mp, C.byref(longest))
+    parts = shim.shim_rows_plan(cpt, tiles, sms, cap, mp, C.byref(longest))
     assert 1 <= parts <= 32 and longest.value <= cap
-    items = (tiles + tw - 1) // tw
-    run = shim.shim_rows_run(items, longest.value, parts, sms)
+    run = shim.shim_rows_run(tiles, longest.value, parts, sms)
     slots = shim.shim_rows_part_slots(cpt, parts, run)
     assert run >= 1
     for part in range(parts):
@@ -38,18 +37,18 @@ def test_every_quad_once_and_shares_agree(shim, k, tiles, cap, mp, tw):
         seen = defaultdict(list)
         taken = 0
         for worker in range(sms // parts * 16):
-            u = min(worker * run, items * quads)
-            end = min(u + run, items * quads)
+            u = min(worker * run, tiles * quads)
+            end = min(u + run, tiles * quads)
             while u < end:
-                item = u // quads
-                stop = min(end, (item + 1) * quads)
+                tile = u // quads
+                stop = min(end, (tile + 1) * quads)
                 taken += stop - u
-                seen[item].append(worker - item * quads // run)
+                seen[tile].append(worker - tile * quads // run)
                 u = stop
-        assert taken == items * quads
-        for item in range(items):
-            assert seen[item] == list(range(shim.shim_rows_shares(item, quads, run)))
-            assert len(seen[item]) <= slots
+        assert taken == tiles * quads
+        for tile in range(tiles):
+            assert seen[tile] == list(range(shim.shim_rows_shares(tile, quads, run)))
+            assert len(seen[tile]) <= slots
 
 
 @pytest.mark.parametrize("cap", [78, 48])  # aligned, byte-addressed
@@ -60,11 +59,11 @@ def test_single_rows_fit_the_scratch_a_runtime_sets_aside(shim, cap):
     for k in (64, 512, 1600, 4096, 5120, 6144, 8192):
         cpt = (k // 64 + 1) // 2
         for tiles in list(range(1, 400)) + list(range(400, 16384, 97)) + [16384]:
-            parts = shim.shim_rows_plan_for(cpt, tiles, 148, cap, 1, 2, C.byref(longest))
+            parts = shim.shim_rows_plan(cpt, tiles, 148, cap, 2, C.byref(longest))
             slots = shim.shim_rows_part_slots(cpt, parts, shim.shim_rows_run(tiles, longest.value, parts, 148))
             assert parts * slots * 2 * tiles * 64 <= 8 << 20, (k, tiles)
 
 
 def test_a_launch_with_more_quads_than_32_bits_is_refused(shim):
     longest = C.c_uint32(0)
-    assert shim.shim_rows_plan_for(136, 0xFFFFFFF, 148, 92, 1, 2, C.byref(longest)) == 0
+    assert shim.shim_rows_plan(136, 0xFFFFFFF, 148, 92, 2, C.byref(longest)) == 0

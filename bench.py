@@ -112,36 +112,8 @@ def secondary_metrics(torch, rt, stack, stream, capi):
 
     out = {}
     with torch.cuda.stream(stream):
-        burst, sustained, source = measured_tensor_peaks()
-        f_gu, f_d = 2.0 * m_max * 2 * inter * hidden, 2.0 * m_max * hidden * inter
-        ms_gu, ms_d = timed(gate_up, m_max, 0, 12, 3), timed(down, m_max, 0, 12, 3)
-        tf_gu, tf_d = f_gu / ms_gu / 1e9, f_d / ms_d / 1e9
-        tf_all = (f_gu + f_d) / (ms_gu + ms_d) / 1e9
-        ms_gu_mis, ms_d_mis = timed(gate_up_mis, m_max, 0, 12, 3), timed(down_mis, m_max, 0, 12, 3)
-        out["prefill_gemm"] = {
-            "workload": "config2-prefill: M=2048, gate+up (K=5120, N=17408 each, one call) and down (K=17408, N=5120); "
-                        "16-byte aligned tensors (the same shapes 2 bytes off a boundary under 'misaligned')",
-            "misaligned": {"gate_up": f_gu / ms_gu_mis / 1e9, "down": f_d / ms_d_mis / 1e9,
-                           "gate_up_down": (f_gu + f_d) / (ms_gu_mis + ms_d_mis) / 1e9},
-            "kernel": "q4_gemm_tc_kernel (tcgen05, in-kernel dequant)", "unit": "TFLOP/s", "dtype": "bf16 x bf16(u4) -> f32",
-            "gate_up": tf_gu, "down": tf_d, "gate_up_down": tf_all, "ms": {"gate_up": ms_gu, "down": ms_d},
-            "peak_burst": burst, "peak_sustained": sustained, "peak_source": source, "peak_datasheet": 2250.0,
-            "frac_of_burst": tf_all / burst, "frac_of_sustained": tf_all / sustained, "frac_of_datasheet": tf_all / 2250.0}
-        # the whole MLP of a layer at M=2048 (fused: gate/up in one launch with the SwiGLU in its epilogue, bf16 hidden
-        # rows straight into the down projection); gate and up must sit at the same offset from a 16-byte boundary, so
-        # the aligned up projections of two layers stand in for an aligned gate/up pair
-        def mlp_of(index, parity):
-            def fn(layer, m, flags):
-                a, b = stack.proj[layer][index], stack.proj[(layer + 1) % layers][index]
-                d = stack.down[(layer * 2 + parity) % layers if layers > 1 else 0]
-                rt.mlp_batch_device(xa.data_ptr(), capi.Q4B_BF16, m, hidden, a.job, b.job, d.job, od.data_ptr(), raw)
-            return fn
-
-        ms_mlp, ms_mlp_mis = timed(mlp_of(stack.up_i, 0), m_max, 0, 8, 3), timed(mlp_of(stack.gate_i, 1), m_max, 0, 8, 3)
-        out["mlp_m2048"] = {"workload": "config2-prefill as one MLP call: M=2048, down(silu(gate x) * (up x)), K=5120, intermediate 17408",
-                            "unit": "TFLOP/s", "value": (f_gu + f_d) / ms_mlp / 1e9, "ms": ms_mlp,
-                            "misaligned": (f_gu + f_d) / ms_mlp_mis / 1e9, "frac_of_burst": (f_gu + f_d) / ms_mlp / 1e9 / burst,
-                            "launches_per_call": 3}
+        # The memory-bound figures first: behind the prompt GEMMs the chip sits at its power cap for a while (1.45-1.65 GHz instead of
+        # 1.965), which made 8 rows of gate/up read 43 us instead of 33.
         # config 0: one 5120 x 5120 matvec (14.7 MB, 2.3 us at the measured HBM peak) -- 48 distinct matrices carved out
         # of lm_head's rows so that no launch finds its weights in L2
         from qwen38_metal_b200.runtime import MappedQ4AffineJob
@@ -175,6 +147,36 @@ def secondary_metrics(torch, rt, stack, stream, capi):
                     cross = m
             sweep[shape]["tensor_wins_from_m"] = cross
         out["small_m_sweep"] = sweep
+        burst, sustained, source = measured_tensor_peaks()
+        f_gu, f_d = 2.0 * m_max * 2 * inter * hidden, 2.0 * m_max * hidden * inter
+        ms_gu, ms_d = timed(gate_up, m_max, 0, 12, 3), timed(down, m_max, 0, 12, 3)
+        tf_gu, tf_d = f_gu / ms_gu / 1e9, f_d / ms_d / 1e9
+        tf_all = (f_gu + f_d) / (ms_gu + ms_d) / 1e9
+        ms_gu_mis, ms_d_mis = timed(gate_up_mis, m_max, 0, 12, 3), timed(down_mis, m_max, 0, 12, 3)
+        out["prefill_gemm"] = {
+            "workload": "config2-prefill: M=2048, gate+up (K=5120, N=17408 each, one call) and down (K=17408, N=5120); "
+                        "16-byte aligned tensors (the same shapes 2 bytes off a boundary under 'misaligned')",
+            "misaligned": {"gate_up": f_gu / ms_gu_mis / 1e9, "down": f_d / ms_d_mis / 1e9,
+                           "gate_up_down": (f_gu + f_d) / (ms_gu_mis + ms_d_mis) / 1e9},
+            "kernel": "q4_gemm_tc_kernel (tcgen05, in-kernel dequant)", "unit": "TFLOP/s", "dtype": "bf16 x bf16(u4) -> f32",
+            "gate_up": tf_gu, "down": tf_d, "gate_up_down": tf_all, "ms": {"gate_up": ms_gu, "down": ms_d},
+            "peak_burst": burst, "peak_sustained": sustained, "peak_source": source, "peak_datasheet": 2250.0,
+            "frac_of_burst": tf_all / burst, "frac_of_sustained": tf_all / sustained, "frac_of_datasheet": tf_all / 2250.0}
+        # the whole MLP of a layer at M=2048 (fused: gate/up in one launch with the SwiGLU in its epilogue, bf16 hidden
+        # rows straight into the down projection); gate and up must sit at the same offset from a 16-byte boundary, so
+        # the aligned up projections of two layers stand in for an aligned gate/up pair
+        def mlp_of(index, parity):
+            def fn(layer, m, flags):
+                a, b = stack.proj[layer][index], stack.proj[(layer + 1) % layers][index]
+                d = stack.down[(layer * 2 + parity) % layers if layers > 1 else 0]
+                rt.mlp_batch_device(xa.data_ptr(), capi.Q4B_BF16, m, hidden, a.job, b.job, d.job, od.data_ptr(), raw)
+            return fn
+
+        ms_mlp, ms_mlp_mis = timed(mlp_of(stack.up_i, 0), m_max, 0, 8, 3), timed(mlp_of(stack.gate_i, 1), m_max, 0, 8, 3)
+        out["mlp_m2048"] = {"workload": "config2-prefill as one MLP call: M=2048, down(silu(gate x) * (up x)), K=5120, intermediate 17408",
+                            "unit": "TFLOP/s", "value": (f_gu + f_d) / ms_mlp / 1e9, "ms": ms_mlp,
+                            "misaligned": (f_gu + f_d) / ms_mlp_mis / 1e9, "frac_of_burst": (f_gu + f_d) / ms_mlp / 1e9 / burst,
+                            "launches_per_call": 3}
     del xa, xh, og, ou, od
     return out
 
@@ -524,7 +526,7 @@ def run_ours(args) -> int:
             "path": ("persistent decode chain (one cooperative launch per token and GPU"
                      + (", peer stores + cross-GPU barriers)" if world > 1 else ")")) if chain is not None
                     else "CUDA graph of per-stage launches + NCCL all-gathers",
-            "roofline": {"bound": "hbm", "kernel": "q4_rows_kernel (per-stage launches, one per projection group; a byte-addressed lm_head: q4_stack_inline_kernel)", "achieved": achieved, "peak": peak,
+            "roofline": {"bound": "hbm", "kernel": "q4_rows_kernel (per-stage launches, one per projection group)", "achieved": achieved, "peak": peak,
                          "peak_source": peak_source, "unit": UNIT, "frac": achieved / peak if peak else None,
                          "frac_of_8TBs": achieved / NOMINAL_HBM_GBS, "launches": prof["launches"],
                          "avg_launch_us": prof["ms"] * 1e3 / max(1, prof["launches"]),

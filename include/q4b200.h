@@ -105,7 +105,7 @@ typedef struct q4b_job {
 
 /* ---- runtime ---- */
 
-/* MetalRuntime::new, src/metal_runtime.rs:642-927. Options are latched from the environment
+/* MetalRuntime::new, src/metal_runtime.rs:642-927. Sets aside about 55 MB of device scratch. Options are latched from the environment
  * once, here (the reference reads QWEN38_* variables, :916-925): Q4B_FORCE_VARIANT. */
 int q4b_runtime_create(int device_ordinal, q4b_runtime **out);
 void q4b_runtime_destroy(q4b_runtime *rt);
@@ -146,9 +146,12 @@ int q4b_matvec_batch(q4b_runtime *rt, const void *x, int x_dtype, uint64_t k, co
                      uint32_t n_jobs, float *const *outputs);
 /* q4_affine_matmul_mapped_batch, src/metal_runtime.rs:3683-3792: x is [m][k] row-major;
  * outputs[i] is [m][jobs[i].output_rows] row-major. Which kernel runs (the reference's dispatcher,
- * src/metal_runtime.rs:24-77, picks by m too): m = 1 the decode kernel; 2 <= m <= 16 the short-batch kernel when
- * k % 512 == 0 and all tensors are 16-byte aligned, else the general streaming kernel (m < 16); from there on the
- * tensor-core GEMM, which rounds activations and dequantised weights to bf16. q4b_describe_dispatch names the choice. */
+ * src/metal_runtime.rs:24-77, picks by m too): up to 15 rows the short-batch kernel, for any byte alignment and any
+ * k % 64 == 0, and 16 rows too when k % 512 == 0 and all tensors are 16-byte aligned; a single byte-addressed row with at
+ * least 131072 outputs (k % 512 == 0) a one-phase launch of the decode chain's kernel; from there on the tensor-core
+ * GEMM, which rounds activations and dequantised weights to bf16 -- a choice of precision, not of speed: at 16 rows
+ * it is already the faster one (Q4B_FLAG_TENSOR). Calls whose output lies over the activation, and shapes that the
+ * short-batch kernel cannot cut, take the streaming kernel. q4b_describe_dispatch names the choice. */
 int q4b_matmul_batch(q4b_runtime *rt, const void *x, int x_dtype, uint64_t m, uint64_t k, const q4b_job *jobs,
                      uint32_t n_jobs, float *const *outputs);
 /* q4_affine_argmax_mapped_batch, src/metal_runtime.rs:3797-3891: tokens[m]; ties -> lowest index. */

@@ -42,13 +42,16 @@
 //
 // Launches are programmatic dependents of whatever runs in front of them: a block requests its first weights and only then waits
 // for the kernel before it, unless that kernel may write them (weights_ahead: the caller holds the address of a shard).
-// What bounds it and what was measured (B200, a graph of calls, one call; in brackets the ring of single chunks with a rolled
-// loop, which issued 162 warp instructions a chunk where 100 will do): 4 rows x 34816 x 5120 24.3 us = 4.1 TB/s (26.0), 4 rows x
-// 248320 x 5120 129 us = 5.5 TB/s (147), 8 fp32 rows x 8192 x 5120 at a byte offset 17.7 us (18.5), one fp32 row x 5120 x 17408 at a
-// byte offset 17.1 us (20.1), 16 rows x 34816 x 5120 63 us (67). Eight rows x 34816 x 5120 take 31.1 us; a form that walked two
-// tiles at a time took 28.8 there and lost everywhere else. Small calls are bound by launch, conversion and the first round
-// trips (2.5 us until the digits are ready, 2 us for the contributions to meet), long ones by the warps' instruction issue.
-// Requesting the second half of the ring only after the activation is out costs 0.6 us in a row of calls and gains nothing.
+// Measured (B200, weights from HBM; in a row of calls, and in brackets with a small kernel of the caller's between them, which cannot let this one
+// start early): 1 row x 5120 x 5120 7.8 us (12.6), 1 x 34816 x 5120 19.5 (24.8), at a byte offset 26.8 (33.4), 4 rows 26.8 (32.9), 8 rows
+// 32.6 = 3.1 TB/s (38.1), 16 rows 63.2 (68.4), 1 fp32 row x 5120 x 17408 at a byte offset 18.1 (24.1), 8 fp32 rows x 8192 x 5120 at a
+// byte offset 17.8 (23.1), 4 rows x 248320 x 5120 141 = 5.1 TB/s (138).
+// What bounds it: 8 rows x 34816 x 5120 issue 205 warp instructions per 1 KB chunk (fixed part included), at 54 % of the issue slots
+// and 40 % of the ALU of sixteen warps an SM, none of which is waiting for memory much: instruction issue and its
+// dependencies. In a call that starts by itself the digits are ready after 7 to 9 us, although they take 2 without weights in flight:
+// the warps stand at their own requests until the memory has taken them. Requesting the second half of the ring after the
+// conversion gives 0.5 to 1.8 us there and costs 0.4 to 1.3 us in a row of calls, requesting nothing before the wait 2 to 3. Two tiles at a
+// time (units of two chunks of two tiles) take 41.9 us for the 8 rows above. Contributions of parts meet in 2 to 3 us.
 #include "q4_decomp.h"
 #include "q4_device.cuh"
 #include "q4_kernels.h"
